@@ -103,7 +103,33 @@ ModCtx make_header(const axhel_ntt_ctx* c, unsigned char* base, uint64_t inv_las
     h.logn = c->logn;
     h.fwd = reinterpret_cast<const ulonglong2*>(base + kHeader);
     h.inv = reinterpret_cast<const ulonglong2*>(base + kHeader + c->n * 16);
+    // Caller-provided tables keep the reference's arithmetic: nothing is
+    // known of their entries.
+    if (c->external) return h;
+    h.arith = c->q < kFpModulusEnd ? 2 : (c->q < kRelaxedModulusEnd ? 1 : 0);
+    if (h.arith == 2) {
+        const auto centred = [&](uint64_t w) { return w > c->q / 2 ? -(double)(c->q - w) : (double)w; };
+        h.fq = (double)c->q;
+        h.fqi = 1.0 / h.fq;
+        h.fninv = centred(ninv);
+        h.fninv_q = h.fninv / h.fq;
+        h.fsroot = centred(sr);
+        h.fsroot_q = h.fsroot / h.fq;
+        // 4 q^2 / 2^64, rounded up
+        const double least = h.fq * h.fq * (4.0 / 18446744073709551616.0) * (1.0 + 1e-12);
+        uint64_t bits;
+        std::memcpy(&bits, &least, sizeof bits);
+        h.lazy_hi = (uint32_t)(bits >> 32);
+        h.ffwd = reinterpret_cast<const double*>(base + kHeader + c->n * 32);
+        h.finv = reinterpret_cast<const double*>(base + kHeader + c->n * 40);
+    }
     return h;
+}
+
+// Bytes of a context made by the library: header, tables, FP64 tables.
+size_t ctx_bytes(uint64_t n, uint64_t q)
+{
+    return kHeader + n * (q < kFpModulusEnd ? 48 : 32);
 }
 
 // Caller-provided tables (the external-table constructor, ntt.cpp:124-133):
@@ -281,7 +307,7 @@ axhel_status_t axhel_cuda_ntt_create_many(uint64_t count, const uint64_t* degree
     size_t total = 0;
     for (size_t k = 0; k < order.size(); ++k) {
         offs[k] = total;
-        total += (kHeader + 2 * order[k]->n * 16 + 255) / 256 * 256;
+        total += (ctx_bytes(order[k]->n, order[k]->q) + 255) / 256 * 256;
     }
     if (total && (e = cudaMalloc(&block, total)) != cudaSuccess) {
         block = nullptr;
@@ -328,8 +354,8 @@ axhel_status_t axhel_cuda_ntt_create_external(uint64_t degree, uint64_t modulus,
     c->q = modulus;
     c->logn = logn;
     cudaGetDevice(&c->device);
-    if ((st = upload(c.get(), fwd, inv, ninv))) return st;
     c->external = true;
+    if ((st = upload(c.get(), fwd, inv, ninv))) return st;
     *out = c.release();
     return AXHEL_OK;
 }
@@ -411,10 +437,48 @@ axhel_status_t collect(const axhel_ntt_t* ntts, uint64_t n_ntts, PassArgs& a, ui
     return AXHEL_OK;
 }
 
+// A lazy forward of fewer residues keeps the integer butterflies: a few limbs
+// are bound by latency, where the FP64 form's longer chain shows (one limb of
+// N = 2^16: 8.1 against 7.3 us, 4 limbs 9.1 against 8.5; 27 limbs of 2^14 9.4
+// against 10.0, 768 limbs of 2^16 499 against 549).
+constexpr uint64_t kLazyFpWords = 3ull << 17;
+
+// A fused chain or product of fewer residues without FP64 moduli keeps the
+// reference's integer butterflies: in a wave that leaves the GPU half empty
+// the relaxed ones' range reductions only lengthen the chain (one limb of
+// N = 2^17: product 16.5 against 15.4 us; 40 limbs of 2^15 32.4 against 41.8).
+constexpr uint64_t kRelaxIntWords = 1ull << 19;
+
+uint64_t fp_moduli(const axhel_ntt_t* ntts, uint64_t n_ntts)
+{
+    uint64_t k = 0;
+    for (uint64_t i = 0; i < n_ntts; ++i) k += !ntts[i]->external && ntts[i]->q < kFpModulusEnd;
+    return k;
+}
+bool fp_any(const axhel_ntt_t* ntts, uint64_t n_ntts) { return fp_moduli(ntts, n_ntts) != 0; }
+
+// Whether a quarter of the moduli or more have FP64 forms.
+bool fp_share(const axhel_ntt_t* ntts, uint64_t n_ntts) { return 4 * fp_moduli(ntts, n_ntts) >= n_ntts; }
+
+// Few enough limbs for the cluster form, whose kernels hold the reference's
+// butterflies only, but the passes in FP64 are faster: from 2^17 residues on
+// (64 limbs of N = 2^12: forward 5.5 against 5.7 us, chain 8.8 against 10.0;
+// 16 of 2^13 5.2 against 5.4, of 2^14 6.0 against 7.8) and from N = 2^15 on
+// (one limb 5.2 against 7.3, chain 9.6 against 12.3; at 2^14 4.9 against 4.5
+// and 9.2 against 8.3).
+// For the fused chains below N = 2^14 the line is twice that (16 limbs of 2^13
+// 9.3 against 8.7 us), likewise where the forward is lazy (8 of 2^14: 12.0
+// against 10.8; 16: 12.6 against 15.0).
+bool fp_passes_win(const axhel_ntt_t* ntts, uint64_t n_ntts, uint32_t logn, uint64_t count, bool fused, bool lazy)
+{
+    const uint64_t words = (fused && logn < 14) || lazy ? 1ull << 18 : 1ull << 17;
+    return ((count << logn) >= words || logn >= 15) && fp_moduli(ntts, n_ntts) == n_ntts;
+}
+
 // Runs the passes of `plan` in order; pass i reads `src` (first pass) or
 // `dst`, writes `dst`.
 axhel_status_t run_plan(bool inverse, const NttPlan& plan, PassArgs a, const uint64_t* src, uint64_t* dst,
-                        uint32_t first_flags, uint32_t last_flags, cudaStream_t s)
+                        uint32_t first_flags, uint32_t last_flags, uint32_t all_flags, cudaStream_t s)
 {
     uint32_t s0 = 0;
     for (int i = 0; i < plan.npass; ++i) {
@@ -423,7 +487,7 @@ axhel_status_t run_plan(bool inverse, const NttPlan& plan, PassArgs a, const uin
         a.dst = dst;
         a.s0 = s0;
         a.tg = (uint32_t)c.tg;
-        a.flags = (i == 0 ? first_flags : 0) | (i == plan.npass - 1 ? (last_flags | kLastPass) : 0);
+        a.flags = all_flags | (i == 0 ? first_flags : 0) | (i == plan.npass - 1 ? (last_flags | kLastPass) : 0);
         cudaError_t e = launch_ntt_pass(inverse, c, a, s);
         if (e != cudaSuccess) return cuda_fail(e, inverse ? "inverse NTT pass" : "forward NTT pass");
         s0 += (uint32_t)c.lg;
@@ -473,8 +537,10 @@ axhel_status_t transform(bool inverse, const axhel_ntt_t* ntts, uint64_t n_ntts,
     // a few limbs: both passes in one launch, one cluster per limb (unless a
     // pass plan was set explicitly for this degree)
     ClusterCfg cc;
+    const bool norm = ((first | last) & (kPostNorm | kPostMul)) != 0;
     if (!plan_overridden(inverse, a.logn) &&
-        cluster_plan(inverse ? kClusterInverse : kClusterForward, a.logn, count, &cc)) {
+        cluster_plan(inverse ? kClusterInverse : kClusterForward, a.logn, count, &cc) &&
+        !(norm && fp_passes_win(ntts, n_ntts, a.logn, count, false, false))) {
         a.src = operand;
         a.dst = result;
         a.s0 = 0;
@@ -486,8 +552,13 @@ axhel_status_t transform(bool inverse, const axhel_ntt_t* ntts, uint64_t n_ntts,
             return cuda_fail(e, inverse ? "inverse NTT (cluster)" : "forward NTT (cluster)");
         // the GPU cannot place the cluster (fewer SMs per GPC): the pass form
     }
-    const NttPlan plan = plan_for(inverse, a.logn, count);
-    return run_plan(inverse, plan, a, operand, result, first, last, S(stream));
+    NttPlan plan = plan_for(inverse, a.logn, count);
+    // normalized output: every pass may work on other representatives; a lazy
+    // forward takes the same kernels' lazy FP64 form for the moduli it covers
+    const bool lazy_fp = !norm && !inverse && (count << a.logn) >= kLazyFpWords && fp_share(ntts, n_ntts);
+    const bool relaxed = (norm || lazy_fp) && plan_relax(plan);
+    const uint32_t relax = relaxed ? (norm ? (uint32_t)kRelaxOut : (uint32_t)kLazyFp) : 0u;
+    return run_plan(inverse, plan, a, operand, result, first, last, relax, S(stream));
 }
 
 axhel_status_t chain(const axhel_ntt_t* ntts, uint64_t n_ntts, uint64_t* result, const uint64_t* operand,
@@ -506,7 +577,8 @@ axhel_status_t chain(const axhel_ntt_t* ntts, uint64_t n_ntts, uint64_t* result,
     const uint32_t logn = c.pass.logn;
     // a few limbs: the whole chain in one launch, one cluster per limb
     ClusterCfg cc;
-    if (!plan_overridden(true, logn) && cluster_plan(kClusterChain, logn, count, &cc)) {
+    if (!plan_overridden(true, logn) && cluster_plan(kClusterChain, logn, count, &cc) &&
+        !fp_passes_win(ntts, n_ntts, logn, count, true, out_f == 4)) {
         c.pass.src = operand;
         c.pass.dst = result;
         c.pass.flags = (in_f == 4 ? (uint32_t)kPreCsub2q : 0u) | (out_f != 4 ? (uint32_t)kPostNorm : 0u);
@@ -519,12 +591,23 @@ axhel_status_t chain(const axhel_ntt_t* ntts, uint64_t n_ntts, uint64_t* result,
         if (e == cudaSuccess) return AXHEL_OK;
         if (!cluster_unschedulable(e)) return cuda_fail(e, "chain (cluster)");
     }
-    const NttPlan inv = plan_for(true, logn, count);
+    NttPlan inv = plan_for(true, logn, count);
+    // the op takes any representative of the inverse's output, and a
+    // normalized forward may work on any
+    const bool relaxable = ((count << logn) >= kRelaxIntWords || fp_any(ntts, n_ntts)) && plan_relax(inv);
+    const uint32_t relax_in = relaxable ? (uint32_t)kRelaxIn : 0u;
+    const uint32_t relax_out = relaxable && out_f != 4 ? (uint32_t)kRelaxOut : 0u;
     // forward passes after the fused one: the inverse's earlier passes, reversed
     NttPlan fwd{};
     fwd.npass = inv.npass;
     for (int i = 0; i < inv.npass; ++i) fwd.pass[i] = inv.pass[inv.npass - 1 - i];
     cudaStream_t s = S(stream);
+    // fused: inverse last pass -> op -> forward first pass.  It holds both
+    // transforms' rounds and the op's operand, so with 16 registers per
+    // thread (LR = 4) it needs 128 registers; 8 (LR = 3) keep it at 76 and
+    // measured 3 % faster at N = 2^16, 768 limbs.
+    PassCfg fc = inv.pass[inv.npass - 1];
+    if (fc.lr > 3 && fc.lg >= 4 && ((uint64_t)fc.tg << (fc.lg - 3)) <= 512) fc.lr = 3;
     // inverse passes before the fused column pass
     uint32_t s0 = 0;
     const uint64_t* src = operand;
@@ -534,24 +617,18 @@ axhel_status_t chain(const axhel_ntt_t* ntts, uint64_t n_ntts, uint64_t* result,
         a.dst = result;
         a.s0 = s0;
         a.tg = (uint32_t)inv.pass[i].tg;
-        a.flags = (i == 0 && in_f == 4) ? (uint32_t)kPreCsub2q : 0u;
+        a.flags = (i == 0 && in_f == 4 ? (uint32_t)kPreCsub2q : 0u) | (relaxable ? (uint32_t)kRelaxOut : 0u);
         cudaError_t e = launch_ntt_pass(true, inv.pass[i], a, s);
         if (e != cudaSuccess) return cuda_fail(e, "chain inverse pass");
         s0 += (uint32_t)inv.pass[i].lg;
         src = result;
     }
-    // fused: inverse last pass -> op -> forward first pass.  It holds both
-    // transforms' rounds and the op's operand, so with 16 registers per
-    // thread (LR = 4) it needs 128 registers; 8 (LR = 3) keep it at 76 and
-    // measured 3 % faster at N = 2^16, 768 limbs.
-    PassCfg fc = inv.pass[inv.npass - 1];
-    if (fc.lr > 3 && fc.lg >= 4 && ((uint64_t)fc.tg << (fc.lg - 3)) <= 512) fc.lr = 3;
     c.pass.src = src;
     c.pass.dst = result;
     c.pass.s0 = s0;
     c.pass.tg = (uint32_t)fc.tg;
     c.pass.flags = (inv.npass == 1 && in_f == 4 ? (uint32_t)kPreCsub2q : 0u) |
-                   (fwd.npass == 1 && out_f != 4 ? (uint32_t)kPostNorm : 0u);
+                   (fwd.npass == 1 && out_f != 4 ? (uint32_t)kPostNorm : 0u) | relax_in | relax_out;
     c.operand = vec;
     c.op = op;
     c.op_factor = 2;
@@ -567,7 +644,8 @@ axhel_status_t chain(const axhel_ntt_t* ntts, uint64_t n_ntts, uint64_t* result,
         a.dst = result;
         a.s0 = f0;
         a.tg = (uint32_t)fwd.pass[i].tg;
-        a.flags = (i == fwd.npass - 1) ? ((uint32_t)kLastPass | (out_f != 4 ? (uint32_t)kPostNorm : 0u)) : 0u;
+        a.flags = (relax_out ? relax_out : (uint32_t)kLazyFp) |
+                  ((i == fwd.npass - 1) ? ((uint32_t)kLastPass | (out_f != 4 ? (uint32_t)kPostNorm : 0u)) : 0u);
         e = launch_ntt_pass(false, fwd.pass[i], a, s);
         if (e != cudaSuccess) return cuda_fail(e, "chain forward pass");
         f0 += (uint32_t)fwd.pass[i].lg;
@@ -594,7 +672,8 @@ axhel_status_t product(const axhel_ntt_t* ntts, uint64_t n_ntts, uint64_t* resul
     const uint32_t logn = c.pass.logn;
     // a few limbs: the whole product in one launch, one cluster per limb
     ClusterCfg cc;
-    if (!plan_overridden(true, logn) && cluster_plan(kClusterProduct, logn, count, &cc)) {
+    if (!plan_overridden(true, logn) && cluster_plan(kClusterProduct, logn, count, &cc) &&
+        !fp_passes_win(ntts, n_ntts, logn, count, true, out_f == 2)) {
         c.pass.src = operand;
         c.pass.dst = result;
         c.pass.flags = out_f != 2 ? (uint32_t)kPostNorm : 0u;
@@ -605,8 +684,18 @@ axhel_status_t product(const axhel_ntt_t* ntts, uint64_t n_ntts, uint64_t* resul
         if (e == cudaSuccess) return AXHEL_OK;
         if (!cluster_unschedulable(e)) return cuda_fail(e, "product (cluster)");
     }
-    const NttPlan inv = plan_for(true, logn, count);
+    NttPlan inv = plan_for(true, logn, count);
     cudaStream_t s = S(stream);
+    // the MulMod takes any representative of the forward's output, and a
+    // normalized inverse may work on any
+    const bool relaxable = ((count << logn) >= kRelaxIntWords || fp_any(ntts, n_ntts)) && plan_relax(inv);
+    const uint32_t relax_in = relaxable ? (uint32_t)kRelaxIn : 0u;
+    const uint32_t relax_out = relaxable && out_f != 2 ? (uint32_t)kRelaxOut : 0u;
+    // fused: forward last pass -> MulMod -> inverse first pass (register depth 3:
+    // the pass holds both transforms' rounds and the multiplicand)
+    PassCfg fc = inv.pass[0];
+    if (fc.lr > 3 && fc.lg >= 4 && ((uint64_t)fc.tg << (fc.lg - 3)) <= 512) fc.lr = 3;
+    if (fc.lr > 3) return fail(AXHEL_ERR_UNSUPPORTED, "no fused product pass for this plan");
     // forward passes before the fused one: the inverse plan's passes npass-1 .. 1
     uint32_t f0 = 0;
     const uint64_t* src = operand;
@@ -616,22 +705,18 @@ axhel_status_t product(const axhel_ntt_t* ntts, uint64_t n_ntts, uint64_t* resul
         a.dst = result;
         a.s0 = f0;
         a.tg = (uint32_t)inv.pass[i].tg;
-        a.flags = 0;
+        a.flags = relaxable ? (uint32_t)kRelaxOut : 0u;
         cudaError_t e = launch_ntt_pass(false, inv.pass[i], a, s);
         if (e != cudaSuccess) return cuda_fail(e, "product forward pass");
         f0 += (uint32_t)inv.pass[i].lg;
         src = result;
     }
-    // fused: forward last pass -> MulMod -> inverse first pass (register depth 3:
-    // the pass holds both transforms' rounds and the multiplicand)
-    PassCfg fc = inv.pass[0];
-    if (fc.lr > 3 && fc.lg >= 4 && ((uint64_t)fc.tg << (fc.lg - 3)) <= 512) fc.lr = 3;
-    if (fc.lr > 3) return fail(AXHEL_ERR_UNSUPPORTED, "no fused product pass for this plan");
     c.pass.src = src;
     c.pass.dst = result;
     c.pass.s0 = 0;
     c.pass.tg = (uint32_t)fc.tg;
-    c.pass.flags = inv.npass == 1 ? ((uint32_t)kLastPass | (out_f != 2 ? (uint32_t)kPostNorm : 0u)) : 0u;
+    c.pass.flags = relax_in | relax_out |
+                   (inv.npass == 1 ? ((uint32_t)kLastPass | (out_f != 2 ? (uint32_t)kPostNorm : 0u)) : 0u);
     c.operand = vec;
     c.op = kChainMul;
     c.op_factor = 4;
@@ -645,7 +730,8 @@ axhel_status_t product(const axhel_ntt_t* ntts, uint64_t n_ntts, uint64_t* resul
         a.dst = result;
         a.s0 = i0;
         a.tg = (uint32_t)inv.pass[i].tg;
-        a.flags = (i == inv.npass - 1) ? ((uint32_t)kLastPass | (out_f != 2 ? (uint32_t)kPostNorm : 0u)) : 0u;
+        a.flags = relax_out |
+                  ((i == inv.npass - 1) ? ((uint32_t)kLastPass | (out_f != 2 ? (uint32_t)kPostNorm : 0u)) : 0u);
         e = launch_ntt_pass(true, inv.pass[i], a, s);
         if (e != cudaSuccess) return cuda_fail(e, "product inverse pass");
         i0 += (uint32_t)inv.pass[i].lg;

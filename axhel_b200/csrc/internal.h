@@ -24,8 +24,22 @@ struct ModCtx {
     uint32_t logn;
     const ulonglong2* fwd;    // N entries {w, floor(w 2^64 / q)}, bit-reversed (ntt-tables.cpp:96-106)
     const ulonglong2* inv;    // N entries, inverse order (ntt-tables.cpp:113-129)
+    // Arithmetic that transforms with normalized output may use (Arith in
+    // ntt_kernels.cuh): 2 = FP64 (q < 2^50), 1 = relaxed integers (q < 2^59),
+    // 0 = the reference's only (wider moduli, caller-provided tables).
+    uint32_t arith;
+    uint32_t lazy_hi;         // FP64: high word of 4 q^2 / 2^64 as a double
+    double fq, fqi;           // FP64: q and 1/q, N^-1 and sroot in (-q/2, q/2] and over q
+    double fninv, fninv_q, fsroot, fsroot_q;
+    const double* ffwd;       // FP64: the twiddles of fwd and inv in (-q/2, q/2] (order: fp_layout.cuh)
+    const double* finv;
 };
-static_assert(sizeof(ModCtx) == 80, "ModCtx layout");
+static_assert(sizeof(ModCtx) == 152, "ModCtx layout");
+
+// Largest moduli of the FP64 and relaxed integer forms: FP64 values within 4q
+// stay below 2^52, relaxed ones below 32q below 2^64.
+constexpr uint64_t kFpModulusEnd = 1ull << 50;
+constexpr uint64_t kRelaxedModulusEnd = 1ull << 59;
 
 constexpr int kMaxInlineMods = 64;
 
@@ -36,6 +50,9 @@ enum PassFlags : uint32_t {
     kLastPass = 4u,      // this pass holds global stage logN-1 (inverse: runs the N^-1 final stage)
     kPreMul = 8u,        // x <- MulMod<4>(x, operand) on load (a dyadic product ahead of an inverse)
     kPostMul = 16u,      // x <- MulMod<4>(x, operand) before the store (a dyadic product after a forward)
+    kRelaxOut = 32u,     // the transform's output is normalized: its stages may work on other representatives
+    kRelaxIn = 64u,      // fused chain / product passes: likewise the transform ahead of the op
+    kLazyFp = 128u,      // lazy forward passes may run in FP64 where the modulus allows
 };
 
 // Geometry of one pass: stages [s0, s0 + lg) of an N = 2^logn transform, on
@@ -79,6 +96,12 @@ cudaError_t launch_chain_pass(const PassCfg& inv_cfg, const ChainArgs& a, cudaSt
 // register depth at most 3).
 cudaError_t launch_product_pass(const PassCfg& cfg, const ChainArgs& a, cudaStream_t s);
 bool pass_supported(const PassCfg& cfg);
+// Whether the pass's kernels hold the relaxed modes: kRelaxOut / kRelaxIn are
+// set on the passes of a call only if all of them do.
+bool pass_relaxable(const PassCfg& cfg);
+// The plan with its passes at the register depth of the relaxed modes, where
+// that fits every pass; false (and `p` as it was) if not.
+bool plan_relax(NttPlan& p);
 
 // Single-launch forms of a few limbs, one thread-block cluster per limb
 // (ntt_cluster.cu): first-pass (transforms) or row (fused chains) stages,
@@ -119,7 +142,8 @@ constexpr size_t kCtxHeaderBytes = 256;
 
 }  // namespace axhel_impl
 
-// One (N, q) transform context: device allocation ModCtx | fwd[N] | inv[N].
+// One (N, q) transform context: device allocation ModCtx | fwd[N] | inv[N],
+// and for the FP64 form ffwd[N] | finv[N].
 struct axhel_ntt_ctx {
     std::atomic<int> refs{1};
     uint64_t n = 0, q = 0, root = 0;

@@ -3,7 +3,10 @@
 // Every routine reproduces, operation for operation, the reference native
 // backend's formula it names, so results are bit-identical including the lazy
 // representatives in [0, 2q) / [0, 4q).  64x64->128 products use
-// __umul64hi / 64-bit mul.lo; no floating point, no tensor cores.
+// __umul64hi / 64-bit mul.lo, no tensor cores.  Where only the residue
+// matters (intermediate values of a transform whose output is reduced to
+// [0, q)), the relaxed and FP64 forms below compute the same residues with
+// other representatives; all of their arithmetic is exact.
 #pragma once
 
 #include <cstdint>
@@ -141,6 +144,94 @@ __device__ __forceinline__ void inv_final_butterfly(uint64_t& x, uint64_t& y, ui
     const uint64_t v = y;
     x = shoup_lazy(gx + v, ninv, ninv_q, q);
     y = shoup_lazy(gx + q2 - v, sr, sr_q, q);
+}
+
+// ------------------------------------------------- relaxed integer forms
+// For transforms whose outputs are reduced to [0, q), so that intermediate
+// values may be any representative.  Bound: the integer multiply pipe, where
+// a high 32-bit product costs two low ones; leaving out the low-by-low term of
+// the quotient and its carries takes the butterfly from 40 to 33 clocks per
+// warp on the register-only probe (q of 58 bits).
+
+// value * w - e * q with e = floor(value * w' / 2^64) - {0, 1, 2}: the terms
+// y1 w'1, floor(y1 w'0 / 2^32) and floor(y0 w'1 / 2^32) only, each floor and
+// the missing y0 w'0 / 2^64 below 1.  The result is in [0, 4q) for any
+// 64-bit value (Shoup's own error is below q, three units more at most).
+__device__ __forceinline__ uint64_t shoup_relaxed(uint64_t v, uint64_t w, uint64_t wq, uint64_t q)
+{
+    uint64_t e;
+    asm("{\n\t"
+        ".reg .u32 a0, a1, b0, b1, u, c, r0, r1;\n\t"
+        "mov.b64 {a0, a1}, %1;\n\t"
+        "mov.b64 {b0, b1}, %2;\n\t"
+        "mul.hi.u32 u, a1, b0;\n\t"
+        "mad.hi.cc.u32 u, a0, b1, u;\n\t"
+        "addc.u32 c, 0, 0;\n\t"
+        "mad.lo.cc.u32 r0, a1, b1, u;\n\t"
+        "madc.hi.u32 r1, a1, b1, c;\n\t"
+        "mov.b64 %0, {r0, r1};\n\t"
+        "}"
+        : "=l"(e)
+        : "l"(v), "l"(wq));
+    return mul_lo_acc(v, w, e, 0 - q);
+}
+
+// ---------------------------------------------------------- FP64 forms
+// For q < 2^50.  Residues are integers held in doubles; every value stays
+// below 2^53 in magnitude and every result is an exact integer.  A butterfly
+// is eight FP64 instructions of two clocks each per warp (the FP64 pipe runs
+// at half the FP32 rate and is otherwise idle here) against 36 clocks of
+// integer multiplies: 17-19 clocks against 40 on the register-only probe.
+
+constexpr double kFpRound = 6755399441055744.0;  // 1.5 * 2^52: adding it rounds to an integer
+constexpr double kFp2p52 = 4503599627370496.0;
+
+__device__ __forceinline__ double as_fp(uint64_t x) { return __longlong_as_double((long long)x); }
+__device__ __forceinline__ uint64_t as_u64(double x) { return (uint64_t)__double_as_longlong(x); }
+
+// Nearest integer to a*b for |a*b| < 2^51 (one rounding).
+__device__ __forceinline__ double fp_quot(double a, double b) { return __dadd_rn(__fma_rn(a, b, kFpRound), -kFpRound); }
+
+// y * w - rint(y * w / q) * q for |y| <= Y q, Y <= 4, |w| <= q/2, wq = w/q.
+// h + l = y w exactly; h - c q is an integer of magnitude below 2^51, so its
+// fma is exact, and so is the sum.  |c - y w / q| <= 1/2 + |y w / q| times the
+// relative error of wq: the result is within q/2 + Y q/16 for wq rounded once
+// (3q/4 at Y = 4) and within q/2 + Y q/8 for wq = w * (1/q rounded).
+__device__ __forceinline__ double fp_mul(double y, double w, double wq, double q)
+{
+    const double h = __dmul_rn(y, w);
+    const double c = fp_quot(y, wq);
+    const double l = __fma_rn(y, w, -h);
+    return __dadd_rn(__fma_rn(-c, q, h), l);
+}
+
+// a * b mod q for |a| <= 3q/4, |b| <= 2q: the quotient from h / q (relative
+// error 2^-52 of at most 1.5 * 2^50), result within 7q/8.
+__device__ __forceinline__ double fp_mulmod(double a, double b, double q, double qi)
+{
+    const double h = __dmul_rn(a, b);
+    const double c = fp_quot(h, qi);
+    const double l = __fma_rn(a, b, -h);
+    return __dadd_rn(__fma_rn(-c, q, h), l);
+}
+
+// x - rint(x / q) * q for |x| < 2^53: within q/2 and a rounding of q/2.
+__device__ __forceinline__ double fp_reduce(double x, double q, double qi) { return __fma_rn(-fp_quot(x, qi), q, x); }
+
+// x < 2^52 as a double, less `off - 2^52`.
+__device__ __forceinline__ double fp_from_u64(uint64_t x, double off)
+{
+    return __dadd_rn(as_fp(x | 0x4330000000000000ull), -off);
+}
+
+// An integer 0 <= x < 2^52 back to 64-bit form.
+__device__ __forceinline__ uint64_t fp_to_u64(double x) { return as_u64(__dadd_rn(x, kFp2p52)) & 0x000fffffffffffffull; }
+
+// The canonical residue of x in (-q, q).
+__device__ __forceinline__ uint64_t fp_canon(double x, double q)
+{
+    const double off = __double2hiint(x) < 0 ? __dadd_rn(q, kFp2p52) : kFp2p52;
+    return as_u64(__dadd_rn(x, off)) & 0x000fffffffffffffull;
 }
 
 }  // namespace axhel_dev

@@ -1,91 +1,75 @@
-// Instantiations and launchers of the NTT pass kernels (ntt_kernels.cuh).
+// Launchers of the NTT pass, chain and product kernels (ntt_kernels.cuh).
 #include <cuda_runtime.h>
 
 #include <mutex>
 
 #include "launch.h"
-#include "ntt_kernels.cuh"
+#include "ntt_table.cuh"
 
 namespace axhel_impl {
 
 namespace {
 
-using PassFn = void (*)(const PassArgs);
-using ChainFn = void (*)(const ChainArgs);
+// Kinds of kernels, for the dynamic shared memory attribute.
+enum FnKind : int { kFnFwd, kFnInv, kFnChain, kFnProduct, kFnFwdMul, kFnInvMul, kFnKinds };
+constexpr int kSmemPlain = 2;  // third "pair" column
+// Two limbs per thread halve the CTAs: only where they still fill the GPU.
+constexpr uint64_t kPairThreadsPerSm = 1024;
 
-constexpr int kMaxLG = 13;
-constexpr int kMaxLR = 5;
-
-struct KernelTable {
-    PassFn fwd[kMaxLG + 1][kMaxLR + 1] = {};
-    PassFn inv[kMaxLG + 1][kMaxLR + 1] = {};
-    PassFn fwd_mul[kMaxLG + 1][kMaxLR + 1] = {};  // with the dyadic product (kPreMul / kPostMul)
-    PassFn inv_mul[kMaxLG + 1][kMaxLR + 1] = {};
-    ChainFn chain[kMaxLG + 1][kMaxLR + 1] = {};
-    ChainFn product[kMaxLG + 1][kMaxLR + 1] = {};
-    bool smem_set[6][kMaxLG + 1][kMaxLR + 1] = {};
-};
-
-template <int LG, int LR>
-void add_one(KernelTable& t)
-{
-    if constexpr (LR <= LG) {
-        t.fwd[LG][LR] = ntt_pass_kernel<false, LG, LR>;
-        t.inv[LG][LR] = ntt_pass_kernel<true, LG, LR>;
-        t.fwd_mul[LG][LR] = ntt_pass_mul_kernel<false, LG, LR>;
-        t.inv_mul[LG][LR] = ntt_pass_mul_kernel<true, LG, LR>;
-        t.chain[LG][LR] = ntt_chain_kernel<LG, LR>;
-        if constexpr (LR <= 3) t.product[LG][LR] = ntt_product_kernel<LG, LR>;
-    }
-}
-
-// Register-stage counts compiled for each group size: LR = LG for tiny groups,
-// otherwise 3, 4 and 5.
-template <int LG>
-void add_lg(KernelTable& t)
-{
-    if constexpr (LG <= 3) {
-        add_one<LG, LG>(t);
-    } else {
-        add_one<LG, 3>(t);
-        add_one<LG, 4>(t);
-        add_one<LG, 5>(t);
-    }
-}
-
-template <int... LG>
-void add_all(KernelTable& t, std::integer_sequence<int, LG...>)
-{
-    (add_lg<LG + 1>(t), ...);
-}
-
-KernelTable& table()
-{
-    static KernelTable t = [] {
-        KernelTable k;
-        add_all(k, std::make_integer_sequence<int, kMaxLG>{});
-        return k;
-    }();
-    return t;
-}
+bool g_smem_set[kFnKinds][2][3][kMaxLG + 1][kMaxLR + 1];
 
 std::mutex g_attr_mu;
 
 size_t smem_bytes(const PassCfg& c) { return (size_t)c.tg * (size_t(1) << c.lg) * sizeof(uint64_t); }
 
 template <class Fn>
-cudaError_t ensure_smem(Fn fn, int kind, const PassCfg& c)
+cudaError_t ensure_smem(Fn fn, FnKind kind, bool relax, int column, const PassCfg& c)
 {
-    const size_t bytes = smem_bytes(c);
+    const size_t bytes = smem_bytes(c) << (column == 1);
     if (bytes <= 48 * 1024) return cudaSuccess;
     std::lock_guard<std::mutex> lk(g_attr_mu);
     // Set to the maximum once per kernel; cheaper than tracking each size.
-    bool& done = table().smem_set[kind][c.lg][c.lr];
+    bool& done = g_smem_set[kind][relax][column][c.lg][c.lr];
     if (done) return cudaSuccess;
     cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(fn),
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (e == cudaSuccess) done = true;
     return e;
+}
+
+// Whether a launch's limbs run two per thread, pairs of the batch's groups of
+// nctx limbs (one per modulus); a last group without a partner costs as much
+// as a pair, so a few odd groups stay single.
+bool pairs(FnKind kind, bool relax, const PassCfg& c, const PassArgs& a)
+{
+    if (kind == kFnFwd && !relax) return false;  // the lazy forms: 333 against 320 us for 768 limbs of 2^16
+    if (!relaxed_compiled(c.lg, c.lr) || (smem_bytes(c) << 1) > 227 * 1024) return false;
+    const uint64_t groups = (a.count + a.nctx - 1) / a.nctx;
+    if (groups < 2 || ((groups & 1) && groups < 7)) return false;
+    return ((a.count << a.logn) >> (c.lr + 1)) >= (uint64_t)sm_count() * kPairThreadsPerSm;
+}
+
+// Launches a pass over its limbs; `pass` is the PassArgs inside the kernel's
+// argument struct `args`.
+template <class Args>
+cudaError_t launch_tiles(const FnTable<void (*)(const Args)>& t, FnKind kind, bool relax, const PassCfg& c,
+                         const Args& args, const PassArgs& pass, cudaStream_t s)
+{
+    const bool plain = (kind == kFnChain || kind == kFnProduct) && !(pass.flags & kRelaxIn);
+    const bool pair = !plain && pairs(kind, relax, c, pass);
+    auto fn = plain ? t.plain[c.lg][c.lr] : t.at[relax][pair][c.lg][c.lr];
+    if (!fn) return cudaErrorInvalidValue;
+    if (pass.count == 0) return cudaSuccess;
+    const cudaError_t e = ensure_smem(fn, kind, relax, plain ? kSmemPlain : pair, c);
+    if (e != cudaSuccess) return e;
+    const uint64_t per_limb = (1ull << (pass.logn - c.lg)) / c.tg;
+    const uint64_t moduli = pass.count < pass.nctx ? pass.count : pass.nctx;
+    const uint64_t groups = (pass.count + moduli - 1) / moduli;
+    const uint64_t gx = ((groups + pair) >> pair) * per_limb;
+    if (pass.count * per_limb > 0x7fffffffull) return cudaErrorInvalidValue;
+    count_launch();
+    fn<<<dim3((unsigned)gx, (unsigned)moduli), (unsigned)c.tg << (c.lg - c.lr), smem_bytes(c) << pair, s>>>(args);
+    return cudaGetLastError();
 }
 
 bool geometry_ok(const PassCfg& c, uint32_t logn, uint32_t lgS)
@@ -107,7 +91,21 @@ bool geometry_ok(const PassCfg& c, uint32_t logn, uint32_t lgS)
 bool pass_supported(const PassCfg& c)
 {
     if (c.lg < 1 || c.lg > kMaxLG || c.lr < 1 || c.lr > kMaxLR) return false;
-    return table().fwd[c.lg][c.lr] != nullptr;
+    return fwd_table().at[0][0][c.lg][c.lr] != nullptr;
+}
+
+bool pass_relaxable(const PassCfg& c) { return relaxed_compiled(c.lg, c.lr); }
+
+bool plan_relax(NttPlan& p)
+{
+    NttPlan r = p;
+    for (int i = 0; i < p.npass; ++i) {
+        PassCfg& c = r.pass[i];
+        c.lr = 3;
+        if (!pass_relaxable(c) || ((uint64_t)c.tg << (c.lg - c.lr)) > (uint64_t)max_threads(c.lr)) return false;
+    }
+    p = r;
+    return true;
 }
 
 cudaError_t launch_ntt_pass(bool inverse, const PassCfg& c, const PassArgs& a, cudaStream_t s)
@@ -116,37 +114,20 @@ cudaError_t launch_ntt_pass(bool inverse, const PassCfg& c, const PassArgs& a, c
     const uint32_t lgS = inverse ? a.s0 : (a.logn - a.s0 - c.lg);
     if (!geometry_ok(c, a.logn, lgS) || (uint32_t)c.tg != a.tg) return cudaErrorInvalidValue;
     const bool mul = (a.flags & (kPreMul | kPostMul)) != 0;
-    PassFn fn = mul ? (inverse ? table().inv_mul[c.lg][c.lr] : table().fwd_mul[c.lg][c.lr])
-                    : (inverse ? table().inv[c.lg][c.lr] : table().fwd[c.lg][c.lr]);
-    cudaError_t e = ensure_smem(fn, (inverse ? 1 : 0) + (mul ? 4 : 0), c);
-    if (e != cudaSuccess) return e;
-    const uint64_t tiles = a.count * ((1ull << (a.logn - c.lg)) / c.tg);
-    if (tiles == 0) return cudaSuccess;
-    if (tiles > 0x7fffffffull) return cudaErrorInvalidValue;
-    const unsigned threads = (unsigned)c.tg << (c.lg - c.lr);
-    count_launch();
+    const FnTable<PassFn>& t = mul ? (inverse ? inv_mul_table() : fwd_mul_table())
+                                   : (inverse ? inv_table() : fwd_table());
+    const FnKind kind = mul ? (inverse ? kFnInvMul : kFnFwdMul) : (inverse ? kFnInv : kFnFwd);
     ProfScope prof(s, "ntt_%s%s_pass lg=%d lr=%d tg=%d", inverse ? "inv" : "fwd", mul ? "_mul" : "", c.lg, c.lr,
                    c.tg);
-    fn<<<(unsigned)tiles, threads, smem_bytes(c), s>>>(a);
-    return cudaGetLastError();
+    return launch_tiles(t, kind, (a.flags & kRelaxOut) != 0, c, a, a, s);
 }
 
 cudaError_t launch_product_pass(const PassCfg& c, const ChainArgs& a, cudaStream_t s)
 {
     if (!pass_supported(c) || c.lr > 3) return cudaErrorInvalidValue;
     if (!geometry_ok(c, a.pass.logn, 0) || (uint32_t)c.tg != a.pass.tg) return cudaErrorInvalidValue;
-    ChainFn fn = table().product[c.lg][c.lr];
-    if (!fn) return cudaErrorInvalidValue;
-    cudaError_t e = ensure_smem(fn, 3, c);
-    if (e != cudaSuccess) return e;
-    const uint64_t tiles = a.pass.count * ((1ull << (a.pass.logn - c.lg)) / c.tg);
-    if (tiles == 0) return cudaSuccess;
-    if (tiles > 0x7fffffffull) return cudaErrorInvalidValue;
-    const unsigned threads = (unsigned)c.tg << (c.lg - c.lr);
-    count_launch();
     ProfScope prof(s, "ntt_product_pass lg=%d lr=%d tg=%d", c.lg, c.lr, c.tg);
-    fn<<<(unsigned)tiles, threads, smem_bytes(c), s>>>(a);
-    return cudaGetLastError();
+    return launch_tiles(product_table(), kFnProduct, (a.pass.flags & kRelaxOut) != 0, c, a, a.pass, s);
 }
 
 cudaError_t launch_chain_pass(const PassCfg& c, const ChainArgs& a, cudaStream_t s)
@@ -154,17 +135,8 @@ cudaError_t launch_chain_pass(const PassCfg& c, const ChainArgs& a, cudaStream_t
     if (!pass_supported(c)) return cudaErrorInvalidValue;
     if (!geometry_ok(c, a.pass.logn, a.pass.logn - c.lg) || (uint32_t)c.tg != a.pass.tg)
         return cudaErrorInvalidValue;
-    ChainFn fn = table().chain[c.lg][c.lr];
-    cudaError_t e = ensure_smem(fn, 2, c);
-    if (e != cudaSuccess) return e;
-    const uint64_t tiles = a.pass.count * ((1ull << (a.pass.logn - c.lg)) / c.tg);
-    if (tiles == 0) return cudaSuccess;
-    if (tiles > 0x7fffffffull) return cudaErrorInvalidValue;
-    const unsigned threads = (unsigned)c.tg << (c.lg - c.lr);
-    count_launch();
     ProfScope prof(s, "ntt_chain_pass lg=%d lr=%d tg=%d", c.lg, c.lr, c.tg);
-    fn<<<(unsigned)tiles, threads, smem_bytes(c), s>>>(a);
-    return cudaGetLastError();
+    return launch_tiles(chain_table(), kFnChain, (a.pass.flags & kRelaxOut) != 0, c, a, a.pass, s);
 }
 
 }  // namespace axhel_impl

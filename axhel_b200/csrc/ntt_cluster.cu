@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(max_threads(LR)) ntt_cluster_kernel(const __gr
     uint64_t v[R];
 
     // second-pass geometry (needed early to prefetch its twiddles)
-    const Tile tB = make_tile<LGB>(INV ? (uint32_t)LGA : 0u, lgtgB, limb, rank);
+    const Tile tB = make_tile<LGB>(INV ? (uint32_t)LGA : 0u, lgtgB, rank);
     uint32_t giB, kB;
     thread_role<LGB, LR>(tB, giB, kB);
     const uint64_t blkB = tile_blk<LGB>(tB, giB);
@@ -254,13 +254,13 @@ __global__ void __launch_bounds__(max_threads(LR)) ntt_cluster_kernel(const __gr
     {
         constexpr int LO_FIRST = round_lo<INV, LGA, LR, 0>();
         constexpr int LO_LAST = round_lo<INV, LGA, LR, NRA - 1>();
-        const Tile t = make_tile<LGA>(INV ? 0u : (uint32_t)LGB, lgtgA, limb, rank);
+        const Tile t = make_tile<LGA>(INV ? 0u : (uint32_t)LGB, lgtgA, rank);
         uint32_t gi, k;
         thread_role<LGA, LR>(t, gi, k);
         const uint64_t blk = tile_blk<LGA>(t, gi);
         load_global<LGA, LR, LO_FIRST>(v, lsrc, t, gi, round_base<LR>(k, LO_FIRST), vec_ok);
         if (a.flags & kPreMul)
-            mul_operand<LGA, LR, LO_FIRST, false>(v, a.operand + (limb << logn), t, gi, k, cx, vec_ok);
+            mul_operand<kExact, LGA, LR, LO_FIRST, false>(v, a.operand + (limb << logn), t, gi, k, cx, vec_ok, 4);
         if constexpr (PRE) {
             PassTw<NRA, LR> pt;
             load_pass_tw<INV, LGA, LR, false>(std::make_integer_sequence<int, NRA>{}, pt, k, blk, 0, n, cx);
@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(max_threads(LR)) ntt_cluster_kernel(const __gr
                 for (int i = 0; i < R; ++i) v[i] = csub_lazy(v[i], q2);
             }
             run_rounds<INV, LGA, LR>(v, scratch + (gi << LGA), k, group_mask<LGA, LR>(t.strided, lgtgA, gi),
-                                     lane_shift(t.strided, lgtgA), blk, 0, n, cx, q, q2, false);
+                                     lane_shift(t.strided, lgtgA), blk, 0, n, cx, false);
         }
         // hand each element to its second-pass owner
         const uint32_t rb = round_base<LR>(k, LO_LAST);
@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(max_threads(LR)) ntt_cluster_kernel(const __gr
 #pragma unroll
         for (int i = 0; i < R; ++i) {
             const uint64_t r = rb + ((uint64_t)i << LO_LAST);
-            const uint64_t p = t.strided ? t.base + gi + (r << t.lgS) : t.base + ((uint64_t)gi << LGA) + r;
+            const uint64_t p = t.strided ? (uint64_t)t.base + gi + (r << t.lgS) : (uint64_t)t.base + (gi << LGA) + r;
             uint32_t owner, off;
             landing_of<INV, LGA>(p, lgchunk, lgtgB, owner, off);
             cl.map_shared_rank(landing, owner)[off] = v[i];
@@ -313,14 +313,14 @@ __global__ void __launch_bounds__(max_threads(LR)) ntt_cluster_kernel(const __gr
         cl.sync();
         load_global<LGB, LR, LO_FIRST>(v, landing, tl, giB, round_base<LR>(kB, LO_FIRST), true);
         run_rounds<INV, LGB, LR>(v, scratch + (giB << LGB), kB, group_mask<LGB, LR>(tB.strided, lgtgB, giB),
-                                 lane_shift(tB.strided, lgtgB), blkB, LGA, n, cx, q, q2, INV);
+                                 lane_shift(tB.strided, lgtgB), blkB, LGA, n, cx, INV);
     }
     if (a.flags & kPostNorm) {
 #pragma unroll
         for (int i = 0; i < R; ++i) v[i] = INV ? csub_lazy(v[i], q) : csub_lazy(csub_lazy(v[i], q2), q);
     }
     if (a.flags & kPostMul)
-        mul_operand<LGB, LR, LO_LAST, false>(v, a.operand + (limb << logn), tB, giB, kB, cx, vec_ok);
+        mul_operand<kExact, LGB, LR, LO_LAST, false>(v, a.operand + (limb << logn), tB, giB, kB, cx, vec_ok, 4);
     store_global<LGB, LR, LO_LAST>(v, ldst, tB, giB, round_base<LR>(kB, LO_LAST), vec_ok);
 }
 
@@ -357,7 +357,7 @@ __device__ __forceinline__ void scatter(const uint64_t (&v)[1 << LR], const Tile
 #pragma unroll
     for (int i = 0; i < (1 << LR); ++i) {
         const uint64_t r = rb + ((uint64_t)i << LO);
-        const uint64_t p = t.strided ? t.base + gi + (r << t.lgS) : t.base + ((uint64_t)gi << LG) + r;
+        const uint64_t p = t.strided ? (uint64_t)t.base + gi + (r << t.lgS) : (uint64_t)t.base + (gi << LG) + r;
         uint32_t owner, off;
         landing_of<TO_COLUMNS, LGR>(p, lgchunk, lgtg_cols, owner, off);
         cl.map_shared_rank(landing, owner)[off] = v[i];
@@ -403,8 +403,8 @@ __global__ void __launch_bounds__(max_threads(LR)) ntt_cluster_fused_kernel(cons
     const uint64_t* lop = c.operand ? c.operand + (limb << logn) : nullptr;
     const bool vec_ok = ((reinterpret_cast<uintptr_t>(a.src) | reinterpret_cast<uintptr_t>(a.dst) |
                           reinterpret_cast<uintptr_t>(c.operand)) & 15) == 0;
-    const Tile tR = make_tile<LGR>(0, lgtgR, limb, rank);
-    const Tile tC = make_tile<LGC>(LGR, lgtgC, limb, rank);
+    const Tile tR = make_tile<LGR>(0, lgtgR, rank);
+    const Tile tC = make_tile<LGC>(LGR, lgtgC, rank);
     uint64_t v[R];
     uint32_t gi, k;
 

@@ -1,0 +1,25 @@
+// The inverse pass kernels with the dyadic product (ntt_kernels.cuh).
+#include "ntt_table.cuh"
+
+namespace axhel_impl {
+
+namespace {
+template <int LG, int LR, bool RELAX, int P>
+struct Get {
+    static constexpr bool compiled = true, has_plain = false;
+    static PassFn fn()
+    {
+        if constexpr (P == 2) return ntt_pass_mul_pair_kernel<true, LG, LR, RELAX>;
+        else if constexpr (LR == 4) return ntt_pass_mul16_kernel<true, LG>;
+        else return ntt_pass_mul_kernel<true, LG, LR, RELAX>;
+    }
+};
+}  // namespace
+
+const FnTable<PassFn>& inv_mul_table()
+{
+    static const FnTable<PassFn> t = make_table<Get, PassFn>(AllGroups{});
+    return t;
+}
+
+}  // namespace axhel_impl

@@ -1,0 +1,66 @@
+// Tables of the compiled pass, chain and product kernels by group size and
+// register depth, one source file per kind (they compile side by side).
+#pragma once
+
+#include <utility>
+
+#include "ntt_kernels.cuh"
+
+namespace axhel_impl {
+
+using PassFn = void (*)(const PassArgs);
+using ChainFn = void (*)(const ChainArgs);
+
+constexpr int kMaxLG = 13;
+constexpr int kMaxLR = 5;
+
+// [1][..]: the kernels launched with kRelaxOut, [..][1]: two limbs per thread;
+// both where relaxed_compiled.
+template <class Fn>
+struct FnTable {
+    Fn at[2][2][kMaxLG + 1][kMaxLR + 1] = {};
+    // Chain and product kernels with the reference's butterflies only, for
+    // launches of a few limbs: those run through their code once, and a
+    // kernel that holds the other arithmetics too takes 13-20 % longer to
+    // fetch it (a chain of one limb of N = 2^16 17.3 against 15.2 us).
+    Fn plain[kMaxLG + 1][kMaxLR + 1] = {};
+};
+
+const FnTable<PassFn>& fwd_table();
+const FnTable<PassFn>& inv_table();
+const FnTable<PassFn>& fwd_mul_table();  // with the dyadic product (kPreMul / kPostMul)
+const FnTable<PassFn>& inv_mul_table();
+const FnTable<ChainFn>& chain_table();
+const FnTable<ChainFn>& product_table();
+
+// Fills a table with Get<LG, LR, RELAX, P>::fn(); P limbs per thread, 0: plain.  Register-stage counts
+// compiled for each group size: LR = LG for tiny groups, otherwise 3, 4 and 5.
+template <template <int, int, bool, int> class Get, class Fn, int LG, int LR>
+void add_one(FnTable<Fn>& t)
+{
+    if constexpr (LR <= LG && Get<LG, LR, false, 1>::compiled) {
+        t.at[0][0][LG][LR] = Get<LG, LR, false, 1>::fn();
+        t.plain[LG][LR] = t.at[0][0][LG][LR];
+        if constexpr (relaxed_compiled(LG, LR) && Get<LG, LR, false, 1>::has_plain)
+            t.plain[LG][LR] = Get<LG, LR, false, 0>::fn();
+        if constexpr (relaxed_compiled(LG, LR)) {
+            t.at[1][0][LG][LR] = Get<LG, LR, true, 1>::fn();
+            t.at[0][1][LG][LR] = Get<LG, LR, false, 2>::fn();
+            t.at[1][1][LG][LR] = Get<LG, LR, true, 2>::fn();
+        }
+    }
+}
+
+template <template <int, int, bool, int> class Get, class Fn, int... I>
+FnTable<Fn> make_table(std::integer_sequence<int, I...>)
+{
+    FnTable<Fn> t;
+    ((I + 1 <= 3 ? add_one<Get, Fn, I + 1, (I + 1 <= 3 ? I + 1 : 3)>(t) : add_one<Get, Fn, I + 1, 3>(t)), ...);
+    ((I + 1 > 3 ? add_one<Get, Fn, I + 1, 4>(t) : void()), ...);
+    ((I + 1 > 3 ? add_one<Get, Fn, I + 1, 5>(t) : void()), ...);
+    return t;
+}
+
+using AllGroups = std::make_integer_sequence<int, kMaxLG>;
+
+}  // namespace axhel_impl

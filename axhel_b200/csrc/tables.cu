@@ -18,10 +18,13 @@
 // the reference does, N^-1, the final-stage scaled root, Barrett and
 // Montgomery constants) and the kernel writes the context header beside the
 // tables, so a context is ready after one launch for any number of (N, q).
+// Moduli below 2^50 get the same twiddles as doubles in (-q/2, q/2] too, for
+// the FP64 butterflies.
 #include <cuda_runtime.h>
 
 #include <cstdint>
 
+#include "fp_layout.cuh"
 #include "internal.h"
 #include "launch.h"
 #include "tables.h"
@@ -67,6 +70,10 @@ __global__ void __launch_bounds__(256) gen_tables_kernel(const __grid_constant__
     const uint64_t w = redc(acc, 0, j.q, j.mninv);           // out of Montgomery form: psi^e mod q
     const uint64_t r = mont_mul(w, j.r2m, j.q, j.mninv);     // w 2^64 mod q
     *out = make_ulonglong2(w, r * j.mninv);                  // Q = (w 2^64 - r) / q
+    if (j.hdr.arith == 2) {
+        double* fout = const_cast<double*>(inv ? j.hdr.finv : j.hdr.ffwd) + (i ? fp_table_pos(inv, i, (uint32_t)n, j.logn) : 0);
+        *fout = (double)(w > (j.q >> 1) ? (int64_t)(w - j.q) : (int64_t)w);
+    }
 }
 
 }  // namespace

@@ -14,7 +14,7 @@ namespace axhel_impl {
 // Montgomery constants of its modulus; the tables follow the header.
 struct TableGenJob {
     ModCtx hdr;
-    unsigned char* base;  // device allocation: header | fwd[n] | inv[n]
+    unsigned char* base;  // device allocation: header | fwd[n] | inv[n] (| ffwd[n] | finv[n])
     uint64_t q;
     uint64_t mninv;       // -q^-1 mod 2^64
     uint64_t r2m;         // 2^128 mod q

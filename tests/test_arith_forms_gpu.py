@@ -1,0 +1,101 @@
+"""The arithmetics of the transform passes (the reference's butterflies, relaxed
+integers, FP64) chosen by modulus width and batch size: every op bit-exact
+against the oracle, for moduli on both sides of each limit in one batch, for
+single limbs, pairs of limbs and an odd last group, on uniform, extreme and
+sparse inputs (zeros and small values need the exact lazy quotient)."""
+import numpy as np
+import pytest
+
+from helpers import dev, dev_empty, host, ptr
+
+pytestmark = pytest.mark.gpu
+
+
+def limit_moduli(oracle, n):
+    """Smallest and largest NTT primes around the limits 2^50 and 2^59, a small and the widest ones."""
+    picks = [(30, 1, 2), (40, 1, 2), (50, 1, 1), (51, 0, 1), (59, 1, 1), (60, 0, 1), (62, 1, 1)]
+    out = []
+    for bits, num, den in picks:
+        q = oracle.find_ntt_prime_near(n, bits, num, den)
+        out.append((q, oracle.find_primitive_root(n, q)))
+    return out
+
+
+def inputs(rng, n, bounds):
+    """Per limb, by turns: uniform, all bound - 1, one nonzero coefficient, small values."""
+    x = np.zeros((len(bounds), n), np.uint64)
+    for i, b in enumerate(bounds):
+        kind = i // 7 % 4
+        if kind == 0:
+            x[i] = rng.integers(0, b, n, dtype=np.uint64)
+        elif kind == 1:
+            x[i] = b - 1
+        elif kind == 2:
+            x[i, rng.integers(n)] = int(rng.integers(1, b, dtype=np.uint64))
+        else:
+            x[i] = rng.integers(0, 3, n, dtype=np.uint64)
+    return x
+
+
+# single limbs, a pair below and above the size from which limbs share a
+# thread, an odd last group; one pass (N <= 2^13 by plan) and two
+@pytest.mark.parametrize("n,polys", [(16, 1), (64, 2), (256, 5), (512, 1), (1024, 2), (4096, 92), (8192, 1), (16384, 23),
+                                     (32768, 2), (65536, 6), (131072, 1)])
+def test_forms_match_oracle(cuda, oracle, n, polys):
+    mods = limit_moduli(oracle, n)
+    L, count = len(mods), len(mods) * polys
+    ntts = cuda.NTT.create_many([(n, q, psi) for q, psi in mods])
+    tabs = [oracle.tables(n, q, psi) for q, psi in mods]
+    rng = np.random.default_rng(n + polys)
+    qs = [mods[i % L][0] for i in range(count)]
+    x4, x2 = inputs(rng, n, [4 * q for q in qs]), inputs(rng, n, [2 * q for q in qs])
+    m4, m2 = inputs(rng, n, [4 * q for q in qs]), inputs(rng, n, [2 * q for q in qs])
+    sc = [(2 * q) // 3 for q, _ in mods]
+    d4, d2, e4, e2, o = dev(x4), dev(x2), dev(m4), dev(m2), dev_empty(count * n)
+    fwd = lambda i, v, f=1: oracle.forward(v, qs[i], tabs[i % L][0], 1, f)
+    inv = lambda i, v, f=1: oracle.inverse(v, qs[i], tabs[i % L][1], tabs[i % L][2], 2, f)
+    red = lambda i, v: oracle.reduce(v, qs[i], 4, 2)
+    ops = {
+        "forward 4": (lambda: cuda.forward_batch(ntts, ptr(o), ptr(d4), count, 4, 4), lambda i: fwd(i, x4[i], 4)),
+        "forward 1": (lambda: cuda.forward_batch(ntts, ptr(o), ptr(d4), count, 4, 1), lambda i: fwd(i, x4[i])),
+        "inverse 1": (lambda: cuda.inverse_batch(ntts, ptr(o), ptr(d2), count, 2, 1), lambda i: inv(i, x2[i])),
+        "inverse 4->1": (lambda: cuda.inverse_batch(ntts, ptr(o), ptr(d4), count, 4, 1),
+                         lambda i: inv(i, red(i, x4[i]))),
+        "inverse 2": (lambda: cuda.inverse_batch(ntts, ptr(o), ptr(d2), count, 2, 2), lambda i: inv(i, x2[i], 2)),
+        "forward mul": (lambda: cuda.forward_mul_batch(ntts, ptr(o), ptr(d4), ptr(e4), count),
+                        lambda i: oracle.mul(fwd(i, x4[i], 4), m4[i], qs[i], 4)),
+        "mul inverse": (lambda: cuda.mul_inverse_batch(ntts, ptr(o), ptr(d4), ptr(e4), count, 1),
+                        lambda i: inv(i, oracle.mul(x4[i], m4[i], qs[i], 4))),
+        "chain mul 1": (lambda: cuda.chain_mul_batch(ntts, ptr(o), ptr(d4), ptr(e2), count, 4, 1),
+                        lambda i: fwd(i, oracle.mul(inv(i, red(i, x4[i]), 2), m2[i], qs[i], 2))),
+        "chain fma 4": (lambda: cuda.chain_fma_batch(ntts, ptr(o), ptr(d2), sc, ptr(e2), count, 2, 4),
+                        lambda i: fwd(i, oracle.fma(inv(i, x2[i], 2), sc[i % L], m2[i], qs[i], 2), 4)),
+        "product 1": (lambda: cuda.product_batch(ntts, ptr(o), ptr(d4), ptr(e4), count, 4, 1),
+                      lambda i: inv(i, oracle.mul(fwd(i, x4[i], 4), m4[i], qs[i], 4))),
+        "product 2": (lambda: cuda.product_batch(ntts, ptr(o), ptr(d4), ptr(e4), count, 4, 2),
+                      lambda i: inv(i, oracle.mul(fwd(i, x4[i], 4), m4[i], qs[i], 4), 2)),
+    }
+    for name, (run, expect) in ops.items():
+        run()
+        got = host(o).reshape(count, n)
+        for i in range(count):
+            np.testing.assert_array_equal(got[i], expect(i), err_msg=f"{name}: limb {i}, q of {qs[i].bit_length()} bits")
+
+
+@pytest.mark.parametrize("bits", [50, 59])
+def test_in_place_and_unaligned(cuda, oracle, bits):
+    """In place, and at 8- and 16-byte aligned addresses (the wide accesses fall back)."""
+    n, polys = 16384, 24
+    q = oracle.find_ntt_prime_near(n, bits, 1, 1)
+    psi = oracle.find_primitive_root(n, q)
+    t = cuda.NTT(n, q, psi)
+    fwd, inv, ninv = oracle.tables(n, q, psi)
+    x = inputs(np.random.default_rng(bits), n, [q] * polys)
+    exp = np.stack([oracle.forward(v, q, fwd, 1, 1) for v in x])
+    for words in (0, 1, 2):
+        buf = dev(np.concatenate([np.zeros(words, np.uint64), x.reshape(-1)]))
+        p = ptr(buf) + 8 * words
+        cuda.forward_batch([t], p, p, polys, 1, 1)
+        np.testing.assert_array_equal(host(buf)[words:].reshape(polys, n), exp, err_msg=f"forward at +{words}")
+        cuda.inverse_batch([t], p, p, polys, 1, 1)
+        np.testing.assert_array_equal(host(buf)[words:].reshape(polys, n), x, err_msg=f"inverse at +{words}")
