@@ -170,7 +170,7 @@ __device__ __forceinline__ void run_elt_tile(const ClassEntry& j, uint64_t limb,
 // registers.  CG: loads bypass L1, for
 // data written by other CTAs of the same launch (the persistent kernel); the
 // per-phase launches read what an earlier launch wrote and load plainly.
-template <int CLS, int LG, int LR, bool CG>
+template <int CLS, int LG, int LR, bool CG, int FORMS>
 __device__ __forceinline__ void run_class_tile(const ClassEntry& c, uint64_t limb, uint64_t tile_in_limb,
                                                uint64_t* sm)
 {
@@ -178,10 +178,10 @@ __device__ __forceinline__ void run_class_tile(const ClassEntry& c, uint64_t lim
     const uint32_t mi = limb_mod(limb, c.nmods);
     const ModCtx* cx = c.ctx[mi];
     if constexpr (CLS == kClsChain) {
-        chain_tile<LG, LR, CG>(c.src, c.dst, c.vec, cx, c.op, c.scalars ? c.scalars[mi] : 0, c.logn, lgtg, limb,
+        chain_tile<LG, LR, CG, FORMS != kFormsExact, FORMS == kFormsRelax>(c.src, c.dst, c.vec, cx, c.op, c.scalars ? c.scalars[mi] : 0, c.logn, lgtg, limb,
                                tile_in_limb, c.flags, sm);
     } else {
-        pass_tile<CLS == kClsInv, LG, LR, CG>(c.src, c.dst, cx, c.logn, c.s0, lgtg, limb, tile_in_limb, c.flags,
+        pass_tile<CLS == kClsInv, LG, LR, CG, false, FORMS != kFormsExact, FORMS == kFormsRelax>(c.src, c.dst, cx, c.logn, c.s0, lgtg, limb, tile_in_limb, c.flags,
                                               sm);
     }
 }
@@ -191,7 +191,7 @@ __device__ __forceinline__ void run_any_tile(const ClassEntry& c, uint64_t limb,
 {
     switch (c.cls_lg) {
 #define AXHEL_TILE_CASE(CLS, LG) \
-    case (CLS << 8) | LG: run_class_tile<CLS, LG, kBatchLR, true>(c, limb, til, sm); break;
+    case (CLS << 8) | LG: run_class_tile<CLS, LG, kBatchLR, true, kFormsExact>(c, limb, til, sm); break;
 #define AXHEL_TILE_CASES(CLS) \
     AXHEL_TILE_CASE(CLS, 5) AXHEL_TILE_CASE(CLS, 6) AXHEL_TILE_CASE(CLS, 7) AXHEL_TILE_CASE(CLS, 8) AXHEL_TILE_CASE(CLS, 9)
     AXHEL_TILE_CASES(kClsFwd)
@@ -294,7 +294,7 @@ constexpr int class_min_blocks()
     return CLS == kClsChain ? 6 : (LR == 4 ? (CLS == kClsInv ? 12 : 16) : kBatchMinBlocks);
 }
 
-template <int CLS, int LG, int LR>
+template <int CLS, int LG, int LR, int FORMS>
 __device__ __forceinline__ void run_class_entry(const ClassEntry& c, uint64_t t, uint64_t* sm)
 {
     const uint64_t lt = t - c.tile0;
@@ -304,12 +304,12 @@ __device__ __forceinline__ void run_class_entry(const ClassEntry& c, uint64_t t,
     if constexpr (CLS == kClsElt)
         run_elt_tile(c, limb, til);
     else
-        run_class_tile<CLS, LG, LR, false>(c, limb, til, sm);
+        run_class_tile<CLS, LG, LR, false, FORMS>(c, limb, til, sm);
 }
 
 // One class launch: CTA b runs the class's tile b (entries in tile order),
 // held to class_min_blocks CTAs per SM.
-template <int CLS, int LG, int LR>
+template <int CLS, int LG, int LR, int FORMS>
 __global__ void __launch_bounds__(kBatchTileWords >> LR, class_min_blocks<CLS, LR>())
     batch_class_kernel(const ClassEntry* __restrict__ ce, uint32_t n_ce)
 {
@@ -320,19 +320,18 @@ __global__ void __launch_bounds__(kBatchTileWords >> LR, class_min_blocks<CLS, L
         const uint32_t mid = (lo + hi) >> 1;
         if (ce[mid].tile0 <= t) lo = mid; else hi = mid;
     }
-    run_class_entry<CLS, LG, LR>(ce[lo], t, sm);
+    run_class_entry<CLS, LG, LR, FORMS>(ce[lo], t, sm);
 }
 
 // A class launch of one entry reads it from the kernel parameters, as the
 // pass kernels read theirs: no dependent load ahead of the tile's data, and
-// its fields stay out of the registers.  Without a CTAs-per-SM bound the
-// compiler settles at 56-64 registers without spills, which measured 4 %
-// faster than the bounded form.
-template <int CLS, int LG, int LR>
-__global__ void __launch_bounds__(kBatchTileWords >> LR) batch_class_one_kernel(const __grid_constant__ ClassEntry one)
+// its fields stay out of the registers.
+template <int CLS, int LG, int LR, int FORMS>
+__global__ void __launch_bounds__(kBatchTileWords >> LR, class_min_blocks<CLS, LR>())
+    batch_class_one_kernel(const __grid_constant__ ClassEntry one)
 {
     __shared__ uint64_t sm[kBatchTileWords + 128];
-    run_class_entry<CLS, LG, LR>(one, blockIdx.x, sm);
+    run_class_entry<CLS, LG, LR, FORMS>(one, blockIdx.x, sm);
 }
 
 }  // namespace axhel_impl
@@ -519,7 +518,11 @@ static void set_specialized(ClassLaunch& L, const BatchJob& b, const std::vector
     a.flags = L.first.flags;
     a.nctx = (uint32_t)ctx.size();
     for (size_t m = 0; m < ctx.size(); ++m) a.ctx[m] = ctx[m];
-    const NttPlan inv = plan_for(true, b.logn, b.count);
+    NttPlan inv = plan_for(true, b.logn, b.count);
+    // the job's passes agree on the arithmetic (batch_build): run them at the
+    // register depth that holds it, or as class launches
+    const bool forms = (L.first.flags & (kRelaxOut | kRelaxIn | kLazyFp)) != 0;
+    if (forms && !plan_relax(inv)) return;
     if (pc.chain) {
         if (inv.npass < 2) return;
         PassCfg fc = inv.pass[inv.npass - 1];
@@ -540,7 +543,8 @@ static void set_specialized(ClassLaunch& L, const BatchJob& b, const std::vector
         L.spec = 2;
         return;
     }
-    const NttPlan pl = pc.inv ? inv : plan_for(false, b.logn, b.count);
+    NttPlan pl = pc.inv ? inv : plan_for(false, b.logn, b.count);
+    if (forms && !plan_relax(pl)) return;
     uint32_t s0 = 0;
     for (int i = 0; i < pl.npass; ++i) {
         if (s0 == pc.s0 && pl.pass[i].lg == (int)pc.lg) {
@@ -567,6 +571,7 @@ axhel_status_t batch_build(const axhel_job_t* jobs, uint64_t n_jobs, unsigned ch
     std::vector<BatchJob> bj(n_jobs);
     std::vector<std::vector<const ModCtx*>> ctxs(n_jobs);
     std::vector<std::vector<uint64_t>> scal(n_jobs);
+    std::vector<uint32_t> n_fp(n_jobs, 0);  // moduli with FP64 forms
     uint64_t done_total = 0;
     for (uint64_t i = 0; i < n_jobs; ++i) {
         const axhel_job_t& J = jobs[i];
@@ -575,6 +580,7 @@ axhel_status_t batch_build(const axhel_job_t* jobs, uint64_t n_jobs, unsigned ch
         const axhel_status_t st = batch_check_job(J, "job " + std::to_string(i), err);
         if (st) return st;
         for (uint32_t m = 0; m < J.n_ntts; ++m) {
+            n_fp[i] += !J.ntts[m]->external && J.ntts[m]->q < kFpModulusEnd;
             ctxs[i].push_back(J.ntts[m]->dctx);
             if (held) held->push_back(J.ntts[m]);
         }
@@ -664,8 +670,23 @@ axhel_status_t batch_build(const axhel_job_t* jobs, uint64_t n_jobs, unsigned ch
         ent_cls[k] = pc.chain ? kClsChain : (pc.inv ? kClsInv : kClsFwd);
         ent_lg[k] = pc.lg;
     }
-    // per (phase, class, pass width): the entries, in order, with their
-    // first tile in that launch's numbering
+    // the arithmetics of every entry, from its job's: a chain's inverse feeds
+    // a MulMod / FMAMod, which takes any representative; lazy forwards run in
+    // FP64 where a quarter of the moduli or more have it
+    std::vector<uint32_t> ent_flags(ent.size(), 0), ent_forms(ent.size(), kFormsExact);
+    for (size_t k = 0; k < ent.size(); ++k) {
+        const BatchJob& b = bj[ent[k].job];
+        if (b.kind >= kJobAdd) continue;
+        const bool chain = b.kind == kJobChainMul || b.kind == kJobChainFma, inverse = ent_cls[k] == kClsInv;
+        const bool lazy_fp = 4 * n_fp[ent[k].job] >= b.nmods;
+        uint32_t& f = ent_flags[k];
+        if (chain && ent_cls[k] == kClsChain) f |= kRelaxIn;
+        if ((chain && inverse) || b.norm) f |= kRelaxOut;
+        else if (!inverse && lazy_fp) f |= kLazyFp;
+        ent_forms[k] = f & kRelaxOut ? kFormsRelax : (f ? kFormsLazy : kFormsExact);
+    }
+    // per (phase, class, pass width, arithmetics): the entries, in order, with
+    // their first tile in that launch's numbering
     std::vector<ClassLaunch> cl;
     std::vector<std::vector<ClassEntry>> cl_ent;
     std::vector<std::vector<uint32_t>> cl_idx;  // the batch entry of each class entry
@@ -686,21 +707,21 @@ axhel_status_t batch_build(const axhel_job_t* jobs, uint64_t n_jobs, unsigned ch
             std::stable_sort(big.begin(), big.end(), [&](uint32_t x, uint32_t y) { return ent_tiles(x) > ent_tiles(y); });
             for (size_t i = 0; i < big.size() && i < kAloneMax; ++i) is_alone[big[i]] = 1;
         }
-        std::map<std::tuple<uint32_t, uint32_t, uint32_t>, size_t> at;
+        std::map<std::tuple<uint32_t, uint32_t, uint32_t, uint32_t>, size_t> at;
         for (uint32_t k = 0; k < (uint32_t)ent.size(); ++k) {
             const BatchEntry& e = ent[k];
             const BatchJob& b = bj[e.job];
-            const uint32_t cls = ent_cls[k], lg = ent_lg[k];
+            const uint32_t cls = ent_cls[k], lg = ent_lg[k], forms = ent_forms[k];
             if (is_alone[k]) {
-                alone.push_back(ClassLaunch{e.phase, cls, lg, 1, nullptr, ent_tiles(k), ClassEntry{}});
+                alone.push_back(ClassLaunch{e.phase, cls, lg, forms, 1, nullptr, ent_tiles(k), ClassEntry{}});
                 alone_idx.push_back(k);
                 continue;
             }
-            const auto key = std::make_tuple(e.phase, cls, lg);
+            const auto key = std::make_tuple(e.phase, cls, lg, forms);
             auto it = at.find(key);
             if (it == at.end()) {
                 it = at.emplace(key, cl.size()).first;
-                cl.push_back(ClassLaunch{e.phase, cls, lg, 0, nullptr, 0, ClassEntry{}});
+                cl.push_back(ClassLaunch{e.phase, cls, lg, forms, 0, nullptr, 0, ClassEntry{}});
                 cl_ent.emplace_back();
                 cl_idx.emplace_back();
             }
@@ -786,6 +807,7 @@ axhel_status_t batch_build(const axhel_job_t* jobs, uint64_t n_jobs, unsigned ch
             // the inverse's last pass holds the N^-1 stage even inside a chain
             if (cls == kClsInv && pc.s0 + ent_lg[k] == b.logn) x.flags |= kLastPass;
         }
+        x.flags |= ent_flags[k];
     }
     std::memcpy(host.data() + targ_off, targ.data(), targ.size() * sizeof(ClassEntry));
     for (size_t c = 0; c < cl.size(); ++c) {
@@ -833,29 +855,36 @@ struct ClassKernel {
 };
 
 // Register depth per class and width: 4 (64 threads per tile) for the
-// 7-stage transform passes, 3 (128 threads) otherwise -- measured per width
-// on the per-phase launches: 4 is 5 % faster at 7 stages, 3 is 8 % faster
-// at 8 stages and 15-22 % faster at 5 and 6.
-template <int CLS, int LG>
+// 7-stage transform passes of the reference's butterflies, 3 (128 threads)
+// otherwise -- measured per width on the per-phase launches: 4 is 5 % faster
+// at 7 stages, 3 is 8 % faster at 8 stages and 15-22 % faster at 5 and 6.
+template <int CLS, int LG, int FORMS>
 ClassKernel class_kernel()
 {
-    constexpr int LR = (CLS == kClsFwd || CLS == kClsInv) && LG == 7 ? 4 : 3;
-    return ClassKernel{batch_class_one_kernel<CLS, LG, LR>, batch_class_kernel<CLS, LG, LR>,
+    constexpr int LR = (CLS == kClsFwd || CLS == kClsInv) && LG == 7 && FORMS == kFormsExact ? 4 : 3;
+    return ClassKernel{batch_class_one_kernel<CLS, LG, LR, FORMS>, batch_class_kernel<CLS, LG, LR, FORMS>,
                        (unsigned)(kBatchTileWords >> LR)};
 }
 
+template <int FORMS>
 ClassKernel pick_class_kernel(uint32_t cls, uint32_t lg)
 {
-    if (cls == kClsElt) return class_kernel<kClsElt, 5>();
-    if (lg < (uint32_t)kBatchMinLG || lg > (uint32_t)kBatchMaxLG) return ClassKernel{};
-    static const ClassKernel table[3][5] = {
-        {class_kernel<kClsFwd, 5>(), class_kernel<kClsFwd, 6>(), class_kernel<kClsFwd, 7>(), class_kernel<kClsFwd, 8>(),
-         class_kernel<kClsFwd, 9>()},
-        {class_kernel<kClsInv, 5>(), class_kernel<kClsInv, 6>(), class_kernel<kClsInv, 7>(), class_kernel<kClsInv, 8>(),
-         class_kernel<kClsInv, 9>()},
-        {class_kernel<kClsChain, 5>(), class_kernel<kClsChain, 6>(), class_kernel<kClsChain, 7>(),
-         class_kernel<kClsChain, 8>(), class_kernel<kClsChain, 9>()}};
+#define AXHEL_CLASS_ROW(CLS)                                                                                 \
+    {class_kernel<CLS, 5, FORMS>(), class_kernel<CLS, 6, FORMS>(), class_kernel<CLS, 7, FORMS>(),            \
+     class_kernel<CLS, 8, FORMS>(), class_kernel<CLS, 9, FORMS>()}
+    static const ClassKernel table[3][5] = {AXHEL_CLASS_ROW(kClsFwd), AXHEL_CLASS_ROW(kClsInv),
+                                            AXHEL_CLASS_ROW(kClsChain)};
+#undef AXHEL_CLASS_ROW
     return cls < 3 ? table[cls][lg - kBatchMinLG] : ClassKernel{};
+}
+
+ClassKernel pick_class_kernel(uint32_t cls, uint32_t lg, uint32_t forms)
+{
+    if (cls == kClsElt) return class_kernel<kClsElt, 5, kFormsExact>();
+    if (lg < (uint32_t)kBatchMinLG || lg > (uint32_t)kBatchMaxLG) return ClassKernel{};
+    return forms == kFormsRelax  ? pick_class_kernel<kFormsRelax>(cls, lg)
+           : forms == kFormsLazy ? pick_class_kernel<kFormsLazy>(cls, lg)
+                                 : pick_class_kernel<kFormsExact>(cls, lg);
 }
 
 }  // namespace
@@ -900,7 +929,7 @@ cudaError_t batch_launch_classes(const std::vector<ClassLaunch>& classes, cudaSt
             const ClassLaunch& L = classes[k];
             if (L.tiles == 0) continue;
             if (L.tiles > 0x7fffffffull) return cudaErrorInvalidValue;
-            const ClassKernel kn = pick_class_kernel(L.cls, L.lg);
+            const ClassKernel kn = pick_class_kernel(L.cls, L.lg, L.forms);
             if (!kn.one) return cudaErrorInvalidValue;
             const int l = (int)((k - i) % nl);
             cudaStream_t ls = l == 0 ? s : lanes->st[l - 1];

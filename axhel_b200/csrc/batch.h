@@ -63,6 +63,10 @@ struct BatchEntry {
 // Tile classes of the per-phase launches: each class runs in a kernel of its
 // own (its own register budget and register depth).
 enum TileClass : uint32_t { kClsFwd = 0, kClsInv = 1, kClsChain = 2, kClsElt = 3 };
+// Which arithmetics a class launch's kernel holds: the reference's butterflies
+// alone (lazy outputs), those of normalized outputs (kRelaxOut), those of a
+// lazy forward (kLazyFp; a chain's fused pass with kRelaxIn alone).
+enum TileForms : uint32_t { kFormsExact = 0, kFormsRelax = 1, kFormsLazy = 2 };
 
 // One entry of a class launch: a (job, phase) with what its tiles read, and
 // its first tile in the launch's numbering.
@@ -81,7 +85,7 @@ struct ClassEntry {
 // One launch of a phase: the tiles of one class and pass width, from
 // every job of the batch, in entry order; or one large entry alone.
 struct ClassLaunch {
-    uint32_t phase, cls, lg, n_ce;
+    uint32_t phase, cls, lg, forms, n_ce;
     const ClassEntry* ce;  // device address, n_ce entries
     uint64_t tiles;
     ClassEntry first;      // host copy of ce[0]: a launch of one entry takes it as a kernel parameter
