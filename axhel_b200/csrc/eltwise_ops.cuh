@@ -15,6 +15,7 @@ using namespace axhel_dev;
 // Each op maps (a, b) -> result for one element.
 
 struct OpAddVV {  // eltwise-add-mod.cpp:15-30
+    static constexpr bool kProduct = false;  // holds a 64 x 64 -> 128 product per element
     static constexpr const char* kName = "add_vv";
     uint64_t q;
     __device__ uint64_t operator()(uint64_t a, uint64_t b) const
@@ -24,6 +25,7 @@ struct OpAddVV {  // eltwise-add-mod.cpp:15-30
     }
 };
 struct OpAddVS {  // eltwise-add-mod.cpp:33-47
+    static constexpr bool kProduct = false;
     static constexpr const char* kName = "add_vs";
     uint64_t q, s;
     __device__ uint64_t operator()(uint64_t a, uint64_t) const
@@ -33,17 +35,20 @@ struct OpAddVS {  // eltwise-add-mod.cpp:33-47
     }
 };
 struct OpSubVV {  // eltwise-sub-mod.cpp:15-30
+    static constexpr bool kProduct = false;
     static constexpr const char* kName = "sub_vv";
     uint64_t q;
     __device__ uint64_t operator()(uint64_t a, uint64_t b) const { return a - b + (a < b ? q : 0); }
 };
 struct OpSubVS {  // eltwise-sub-mod.cpp:33-47
+    static constexpr bool kProduct = false;
     static constexpr const char* kName = "sub_vs";
     uint64_t q, s;
     __device__ uint64_t operator()(uint64_t a, uint64_t) const { return a - s + (a < s ? q : 0); }
 };
 template <int F>
 struct OpMul {  // EltwiseMulModNative<F>, eltwise-mul-mod.cpp:18-63
+    static constexpr bool kProduct = true;
     static constexpr const char* kName = "mul";
     uint64_t q, mu;
     uint32_t shift;
@@ -54,6 +59,7 @@ struct OpMul {  // EltwiseMulModNative<F>, eltwise-mul-mod.cpp:18-63
 };
 template <int F, bool ADD>
 struct OpFma {  // EltwiseFMAModNative<F>, eltwise-fma-mod.cpp:18-78 (b = op3[i] when ADD)
+    static constexpr bool kProduct = true;
     static constexpr const char* kName = "fma";
     uint64_t q, mu, s;  // s already reduced by ReduceInput<F>
     uint32_t shift;
@@ -69,6 +75,7 @@ struct OpFma {  // EltwiseFMAModNative<F>, eltwise-fma-mod.cpp:18-78 (b = op3[i]
 };
 template <int KIND>
 struct OpReduce {  // EltwiseReduceModNative branches, eltwise-reduce-mod.cpp:32-128
+    static constexpr bool kProduct = false;
     static constexpr const char* kName = "reduce";
     uint64_t q, mu;
     uint32_t shift;

@@ -271,3 +271,22 @@ def test_unaligned_large_all_ops(cuda, oracle, in_place):
         do = da if in_place else dev_empty(n + 1, fill=0)
         run(ptr(do, 1), ptr(da, 1), ptr(db, 1), ptr(dc, 1))
         np.testing.assert_array_equal(host(do, n + 1)[1:], want(), err_msg=f"op {k} in_place={in_place}")
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 4, 5, 7, 8, 9, 1027, 4099])
+@pytest.mark.parametrize("offsets", [(0, 0, 0), (1, 1, 1), (2, 2, 2), (3, 3, 3), (0, 1, 0), (2, 0, 2), (1, 1, 3)])
+def test_product_alignments(cuda, oracle, n, offsets):
+    """MulMod and FMAMod at every offset from a 32-byte boundary, shared by the operands and not."""
+    q, f = 576460752303423433, 4
+    rng = np.random.default_rng(n)
+    a, b = (rng.integers(0, f * q, n, dtype=np.uint64) for _ in range(2))
+    pad = lambda v, o: dev(np.concatenate([np.zeros(o, np.uint64), v, np.zeros(4, np.uint64)]))
+    for name, run, exp in (
+            ("mul", lambda r, x, y: cuda.mul(r, x, y, n, q, f), oracle.mul(a, b, q, f)),
+            ("fma", lambda r, x, y: cuda.fma(r, x, q - 3, y, n, q, f), oracle.fma(a, q - 3, b, q, f)),
+            ("fma, no addend", lambda r, x, y: cuda.fma(r, x, q - 3, 0, n, q, f), oracle.fma(a, q - 3, None, q, f))):
+        o, da, db = pad(np.zeros(n, np.uint64), offsets[0]), pad(a, offsets[1]), pad(b, offsets[2])
+        run(ptr(o, offsets[0]), ptr(da, offsets[1]), ptr(db, offsets[2]))
+        got = host(o)
+        np.testing.assert_array_equal(got[offsets[0]:offsets[0] + n], exp, err_msg=name)
+        assert not got[:offsets[0]].any() and not got[offsets[0] + n:].any(), f"{name}: wrote outside"
