@@ -267,7 +267,8 @@ cudaError_t eltwise_reduce(uint64_t* r, const uint64_t* a, uint64_t n, uint64_t 
 
 struct ModConst {
     uint64_t q, mu;
-    uint32_t shift, pad;
+    uint32_t shift, fp;  // fp: q < 2^50, the FP64 form
+    double fq, fqi;
 };
 struct TensorArgs {
     uint64_t *r0, *r1, *r2;
@@ -282,12 +283,37 @@ struct TensorArgs {
 // with EltwiseMulMod<F> / EltwiseAddMod semantics (canonical results, so the
 // middle term's evaluation order is free); the trailing EltwiseReduceMod(4,1)
 // is the identity on these canonical values.
+//
+// HBM-bound (56 bytes per element) while the products keep up: three Barrett
+// products are about 180 clocks of the multiply pipe per warp and element, of
+// the 300 or so that its bytes take.  Moduli below 2^50 take about 40 FP64
+// instructions of two clocks instead.  64 pairs x 16 limbs (40-55 bits) of
+// N = 2^15: factor 1 305 to 285 us (6.6 TB/s), factor 4 360 to 288.
+template <int F>
+__device__ __forceinline__ void tensor_fp(uint64_t c0, uint64_t c1, uint64_t d0, uint64_t d1, uint64_t& r0,
+                                          uint64_t& r1, uint64_t& r2, double q, double qi)
+{
+    // factor 1: within q; else within 2q, and the first factors brought to q/2
+    const double off = F == 1 ? kFp2p52 : __fma_rn(2.0, q, kFp2p52);
+    double x0 = fp_from_u64(c0, off), x1 = fp_from_u64(c1, off);
+    const double y0 = fp_from_u64(d0, off), y1 = fp_from_u64(d1, off);
+    if constexpr (F != 1) {
+        x0 = fp_reduce(x0, q, qi);
+        x1 = fp_reduce(x1, q, qi);
+    }
+    const double p0 = fp_mulmod(x0, y0, q, qi), p2 = fp_mulmod(x1, y1, q, qi);
+    const double p1 = fp_mulmod(fp_reduce(__dadd_rn(x0, x1), q, qi), __dadd_rn(y0, y1), q, qi);
+    r0 = fp_canon(p0, q);
+    r2 = fp_canon(p2, q);
+    r1 = fp_canon(fp_reduce(__dadd_rn(__dadd_rn(p1, -p0), -p2), q, qi), q);
+}
+
 template <int F>
 __global__ void __launch_bounds__(256) tensor_product_kernel(const __grid_constant__ TensorArgs a)
 {
     // grid: x = chunks of one limb, y = limb.  Two elements per thread step.
     const uint64_t limb = blockIdx.y;
-    const ModConst mc = a.m[limb % a.nmod];
+    const ModConst& mc = a.m[limb % a.nmod];
     const uint64_t q = mc.q;
     const OpMul<1> mul{q, mc.mu, mc.shift};  // on inputs already reduced to [0, q)
     const OpAddVV add{q};
@@ -313,8 +339,13 @@ __global__ void __launch_bounds__(256) tensor_product_kernel(const __grid_consta
         const ulonglong2 y0 = *reinterpret_cast<const ulonglong2*>(a.d0 + off + e);
         const ulonglong2 y1 = *reinterpret_cast<const ulonglong2*>(a.d1 + off + e);
         uint64_t r[2][3];
-        three(x0.x, x1.x, y0.x, y1.x, r[0][0], r[0][1], r[0][2]);
-        three(x0.y, x1.y, y0.y, y1.y, r[1][0], r[1][1], r[1][2]);
+        if (mc.fp) {
+            tensor_fp<F>(x0.x, x1.x, y0.x, y1.x, r[0][0], r[0][1], r[0][2], mc.fq, mc.fqi);
+            tensor_fp<F>(x0.y, x1.y, y0.y, y1.y, r[1][0], r[1][1], r[1][2], mc.fq, mc.fqi);
+        } else {
+            three(x0.x, x1.x, y0.x, y1.x, r[0][0], r[0][1], r[0][2]);
+            three(x0.y, x1.y, y0.y, y1.y, r[1][0], r[1][1], r[1][2]);
+        }
         const ulonglong2 o0 = make_ulonglong2(r[0][0], r[1][0]);
         const ulonglong2 o1 = make_ulonglong2(r[0][1], r[1][1]);
         const ulonglong2 o2 = make_ulonglong2(r[0][2], r[1][2]);
@@ -337,12 +368,16 @@ cudaError_t tensor_product(uint64_t* r0, uint64_t* r1, uint64_t* r2, const uint6
     for (uint64_t i = 0; i < nmod; ++i) {
         a.m[i].q = moduli[i];
         barrett_params(moduli[i], &a.m[i].mu, &a.m[i].shift);
+        a.m[i].fp = moduli[i] < kFpModulusEnd;
+        a.m[i].fq = (double)moduli[i];
+        a.m[i].fqi = 1.0 / a.m[i].fq;
     }
     if (n == 0 || count == 0) return cudaSuccess;
     const int threads = 256;
     uint64_t bx = (n / 2 + threads - 1) / threads;
-    // enough CTAs for ~8 per SM in total, at least one per limb
-    uint64_t want = ((uint64_t)sm_count() * 8 + count - 1) / count;
+    // 64 CTAs per SM in total, at least one per limb (8: 305 us, 64: 293, one
+    // chunk per CTA: 326, on the shape above)
+    uint64_t want = ((uint64_t)sm_count() * 64 + count - 1) / count;
     if (want < 1) want = 1;
     if (bx > want) bx = want;
     const dim3 grid((unsigned)bx, (unsigned)count);

@@ -205,8 +205,9 @@ __device__ __forceinline__ double fp_mul(double y, double w, double wq, double q
     return __dadd_rn(__fma_rn(-c, q, h), l);
 }
 
-// a * b mod q for |a| <= 3q/4, |b| <= 2q: the quotient from h / q (relative
-// error 2^-52 of at most 1.5 * 2^50), result within 7q/8.
+// a * b mod q for |a b| <= 2 q^2, |a|, |b| <= 4q: the quotient from h / q, with
+// a relative error of 2^-52, so the result is within q/2 + |a b| / 4q (7q/8 for
+// |a| <= 3q/4, |b| <= 2q; q at most).
 __device__ __forceinline__ double fp_mulmod(double a, double b, double q, double qi)
 {
     const double h = __dmul_rn(a, b);

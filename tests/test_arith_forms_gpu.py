@@ -99,3 +99,24 @@ def test_in_place_and_unaligned(cuda, oracle, bits):
         np.testing.assert_array_equal(host(buf)[words:].reshape(polys, n), exp, err_msg=f"forward at +{words}")
         cuda.inverse_batch([t], p, p, polys, 1, 1)
         np.testing.assert_array_equal(host(buf)[words:].reshape(polys, n), x, err_msg=f"inverse at +{words}")
+
+
+@pytest.mark.parametrize("factor", [1, 2, 4])
+def test_tensor_forms(cuda, oracle, factor):
+    """The tensor product on moduli around the FP64 limit (any modulus, prime or not), uniform and extreme inputs."""
+    n, qs = 1026, [17, (1 << 30) - 35, (1 << 50) - 27, (1 << 50) + 55, (1 << 61) + 15]
+    rng = np.random.default_rng(factor)
+    count = 4 * 7 * len(qs)
+    bounds = [factor * qs[i % len(qs)] for i in range(count)]
+    x = [inputs(rng, n, bounds) for _ in range(4)]
+    d = [dev(v) for v in x]
+    r = [dev_empty(count * n) for _ in range(3)]
+    cuda.tensor_product(*[ptr(t) for t in (*r, *d)], n, count, qs, factor)
+    got = [host(t).reshape(count, n) for t in r]
+    for i in range(count):
+        q = qs[i % len(qs)]
+        c0, c1, d0, d1 = (v[i] for v in x)
+        mul = lambda a, b: oracle.mul(a, b, q, factor)
+        exp = (mul(c0, d0), oracle.add(mul(c0, d1), mul(c1, d0), q), mul(c1, d1))
+        for k in range(3):
+            np.testing.assert_array_equal(got[k][i], exp[k], err_msg=f"limb {i} output {k} q={q}")
