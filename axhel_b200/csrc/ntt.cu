@@ -16,20 +16,20 @@ constexpr int kSmemPlain = 2;  // third "pair" column
 // Two limbs per thread halve the CTAs: only where they still fill the GPU.
 constexpr uint64_t kPairThreadsPerSm = 1024;
 
-bool g_smem_set[kFnKinds][2][3][kMaxLG + 1][kMaxLR + 1];
+bool g_smem_set[kFnKinds][2][3][2][kMaxLG + 1][kMaxLR + 1];
 
 std::mutex g_attr_mu;
 
 size_t smem_bytes(const PassCfg& c) { return (size_t)c.tg * (size_t(1) << c.lg) * sizeof(uint64_t); }
 
 template <class Fn>
-cudaError_t ensure_smem(Fn fn, FnKind kind, bool relax, int column, const PassCfg& c)
+cudaError_t ensure_smem(Fn fn, FnKind kind, bool relax, int column, bool row, const PassCfg& c)
 {
     const size_t bytes = smem_bytes(c) << (column == 1);
     if (bytes <= 48 * 1024) return cudaSuccess;
     std::lock_guard<std::mutex> lk(g_attr_mu);
     // Set to the maximum once per kernel; cheaper than tracking each size.
-    bool& done = g_smem_set[kind][relax][column][c.lg][c.lr];
+    bool& done = g_smem_set[kind][relax][column][row][c.lg][c.lr];
     if (done) return cudaSuccess;
     cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(fn),
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
@@ -53,14 +53,14 @@ bool pairs(FnKind kind, bool relax, const PassCfg& c, const PassArgs& a)
 // argument struct `args`.
 template <class Args>
 cudaError_t launch_tiles(const FnTable<void (*)(const Args)>& t, FnKind kind, bool relax, const PassCfg& c,
-                         const Args& args, const PassArgs& pass, cudaStream_t s)
+                         const Args& args, const PassArgs& pass, bool row, cudaStream_t s)
 {
     const bool plain = (kind == kFnChain || kind == kFnProduct) && !(pass.flags & kRelaxIn);
     const bool pair = !plain && pairs(kind, relax, c, pass);
-    auto fn = plain ? t.plain[c.lg][c.lr] : t.at[relax][pair][c.lg][c.lr];
+    auto fn = plain ? t.plain[c.lg][c.lr] : t.at[relax][pair][row][c.lg][c.lr];
     if (!fn) return cudaErrorInvalidValue;
     if (pass.count == 0) return cudaSuccess;
-    const cudaError_t e = ensure_smem(fn, kind, relax, plain ? kSmemPlain : pair, c);
+    const cudaError_t e = ensure_smem(fn, kind, relax, plain ? kSmemPlain : pair, row, c);
     if (e != cudaSuccess) return e;
     const uint64_t per_limb = (1ull << (pass.logn - c.lg)) / c.tg;
     const uint64_t moduli = pass.count < pass.nctx ? pass.count : pass.nctx;
@@ -91,7 +91,7 @@ bool geometry_ok(const PassCfg& c, uint32_t logn, uint32_t lgS)
 bool pass_supported(const PassCfg& c)
 {
     if (c.lg < 1 || c.lg > kMaxLG || c.lr < 1 || c.lr > kMaxLR) return false;
-    return fwd_table().at[0][0][c.lg][c.lr] != nullptr;
+    return fwd_table().at[0][0][1][c.lg][c.lr] != nullptr;
 }
 
 bool pass_relaxable(const PassCfg& c) { return relaxed_compiled(c.lg, c.lr); }
@@ -119,7 +119,7 @@ cudaError_t launch_ntt_pass(bool inverse, const PassCfg& c, const PassArgs& a, c
     const FnKind kind = mul ? (inverse ? kFnInvMul : kFnFwdMul) : (inverse ? kFnInv : kFnFwd);
     ProfScope prof(s, "ntt_%s%s_pass lg=%d lr=%d tg=%d", inverse ? "inv" : "fwd", mul ? "_mul" : "", c.lg, c.lr,
                    c.tg);
-    return launch_tiles(t, kind, (a.flags & kRelaxOut) != 0, c, a, a, s);
+    return launch_tiles(t, kind, (a.flags & kRelaxOut) != 0, c, a, a, lgS == 0, s);
 }
 
 cudaError_t launch_product_pass(const PassCfg& c, const ChainArgs& a, cudaStream_t s)
@@ -127,7 +127,7 @@ cudaError_t launch_product_pass(const PassCfg& c, const ChainArgs& a, cudaStream
     if (!pass_supported(c) || c.lr > 3) return cudaErrorInvalidValue;
     if (!geometry_ok(c, a.pass.logn, 0) || (uint32_t)c.tg != a.pass.tg) return cudaErrorInvalidValue;
     ProfScope prof(s, "ntt_product_pass lg=%d lr=%d tg=%d", c.lg, c.lr, c.tg);
-    return launch_tiles(product_table(), kFnProduct, (a.pass.flags & kRelaxOut) != 0, c, a, a.pass, s);
+    return launch_tiles(product_table(), kFnProduct, (a.pass.flags & kRelaxOut) != 0, c, a, a.pass, true, s);
 }
 
 cudaError_t launch_chain_pass(const PassCfg& c, const ChainArgs& a, cudaStream_t s)
@@ -136,7 +136,7 @@ cudaError_t launch_chain_pass(const PassCfg& c, const ChainArgs& a, cudaStream_t
     if (!geometry_ok(c, a.pass.logn, a.pass.logn - c.lg) || (uint32_t)c.tg != a.pass.tg)
         return cudaErrorInvalidValue;
     ProfScope prof(s, "ntt_chain_pass lg=%d lr=%d tg=%d", c.lg, c.lr, c.tg);
-    return launch_tiles(chain_table(), kFnChain, (a.pass.flags & kRelaxOut) != 0, c, a, a.pass, s);
+    return launch_tiles(chain_table(), kFnChain, (a.pass.flags & kRelaxOut) != 0, c, a, a.pass, true, s);
 }
 
 }  // namespace axhel_impl

@@ -4,14 +4,14 @@
 namespace axhel_impl {
 
 namespace {
-template <int LG, int LR, bool RELAX, int P>
+template <int LG, int LR, bool RELAX, int P, int SHAPE>
 struct Get {
-    static constexpr bool compiled = true, has_plain = false;
+    static constexpr bool compiled = true, has_plain = false, shaped = true;
     static PassFn fn()
     {
-        if constexpr (P == 2) return ntt_pass_mul_pair_kernel<false, LG, LR, RELAX>;
-        else if constexpr (LR == 4) return ntt_pass_mul16_kernel<false, LG>;
-        else return ntt_pass_mul_kernel<false, LG, LR, RELAX>;
+        if constexpr (P == 2) return ntt_pass_mul_pair_kernel<false, LG, LR, RELAX, SHAPE>;
+        else if constexpr (LR == 4) return ntt_pass_mul16_kernel<false, LG, SHAPE>;
+        else return ntt_pass_mul_kernel<false, LG, LR, RELAX, SHAPE>;
     }
 };
 }  // namespace

@@ -4,14 +4,14 @@
 namespace axhel_impl {
 
 namespace {
-template <int LG, int LR, bool RELAX, int P>
+template <int LG, int LR, bool RELAX, int P, int SHAPE>
 struct Get {
-    static constexpr bool compiled = true, has_plain = false;
+    static constexpr bool compiled = true, has_plain = false, shaped = true;
     static PassFn fn()
     {
-        if constexpr (P == 2) return ntt_pass_pair_kernel<true, LG, LR, RELAX>;
-        else if constexpr (LR == 4) return ntt_pass16_kernel<true, LG>;
-        else return ntt_pass_kernel<true, LG, LR, RELAX>;
+        if constexpr (P == 2) return ntt_pass_pair_kernel<true, LG, LR, RELAX, SHAPE>;
+        else if constexpr (LR == 4) return ntt_pass16_kernel<true, LG, SHAPE>;
+        else return ntt_pass_kernel<true, LG, LR, RELAX, SHAPE>;
     }
 };
 }  // namespace

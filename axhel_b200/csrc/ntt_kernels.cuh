@@ -138,13 +138,13 @@ struct Tile {
 // Tile `tile_in_limb` of a limb for a pass with group stride 2^lgS and
 // 2^lgtg groups per tile.
 template <int LG>
-__device__ __forceinline__ Tile make_tile(uint32_t lgS, uint32_t lgtg, uint64_t tile_in_limb)
+__device__ __forceinline__ Tile make_tile(uint32_t lgS, uint32_t lgtg, uint64_t tile_in_limb, bool strided)
 {
     Tile t;
     t.g0 = (uint32_t)tile_in_limb << lgtg;
     t.lgS = lgS;
     t.lgtg = lgtg;
-    t.strided = lgS != 0;
+    t.strided = strided;
     if (t.strided) {
         const uint32_t blk = t.g0 >> lgS, col = t.g0 & ((1u << lgS) - 1);
         t.base = (blk << (LG + lgS)) + col;
@@ -153,6 +153,17 @@ __device__ __forceinline__ Tile make_tile(uint32_t lgS, uint32_t lgtg, uint64_t 
     }
     return t;
 }
+
+template <int LG>
+__device__ __forceinline__ Tile make_tile(uint32_t lgS, uint32_t lgtg, uint64_t tile_in_limb)
+{
+    return make_tile<LG>(lgS, lgtg, tile_in_limb, lgS != 0);
+}
+
+// Which tiles a kernel is compiled for: strided columns, contiguous rows, or
+// either.  One kind alone is half the code: fewer registers, and a launch of
+// a few limbs, which runs through its code once, fetches less of it.
+enum TileShape : int { kAnyTiles = 0, kColumnTiles = 1, kRowTiles = 2 };
 
 template <int LG>
 __device__ __forceinline__ uint32_t tile_blk(const Tile& t, uint32_t gi)
@@ -807,7 +818,7 @@ __device__ __forceinline__ void mul_operand(uint64_t (&v)[1 << LR], const uint64
 // residues, and with one limb per thread twiddles were two thirds of its
 // wavefronts (profiled at N = 2^16: 78-86 % of the pipe's cycles); two limbs
 // of a modulus share every twiddle, its address and the barriers.
-template <int MODE, bool INV, int LG, int LR, bool CG, bool MUL, int P>
+template <int MODE, bool INV, int LG, int LR, bool CG, bool MUL, int P, int SHAPE>
 __device__ __forceinline__ void pass_tile_as(const uint64_t* src, uint64_t* dst, const ModCtx* cx, uint32_t logn,
                                              uint32_t s0, uint32_t lgtg, uint64_t limb, uint64_t lstep,
                                              uint64_t tile_in_limb, uint32_t flags, uint64_t* sm,
@@ -817,8 +828,8 @@ __device__ __forceinline__ void pass_tile_as(const uint64_t* src, uint64_t* dst,
     constexpr int NR = num_rounds<LG, LR>();
     constexpr int LO_FIRST = round_lo<INV, LG, LR, 0>();
     constexpr int LO_LAST = round_lo<INV, LG, LR, NR - 1>();
-    const uint32_t lgS = INV ? s0 : (logn - s0 - LG);
-    const Tile t = make_tile<LG>(lgS, lgtg, tile_in_limb);
+    const uint32_t lgS = SHAPE == kRowTiles ? 0u : (INV ? s0 : (logn - s0 - LG));
+    const Tile t = make_tile<LG>(lgS, lgtg, tile_in_limb, SHAPE == kColumnTiles || (SHAPE == kAnyTiles && lgS != 0));
     const uint32_t n = 1u << logn;
     const uint64_t* lsrc = src + (limb << logn);
     uint64_t* ldst = dst + (limb << logn);
@@ -849,7 +860,7 @@ __device__ __forceinline__ void pass_tile_as(const uint64_t* src, uint64_t* dst,
                                                         vec_ok, 4);
     }
     run_rounds<INV, LG, LR, MODE, P>(v, sm, k, group_slot<LG, LR>(t.strided, lgtg, gi),
-                                     lane_shift(t.strided, lgtg), 1u << (LG + lgtg), blk, s0, n, cx, lgS == 0, last);
+                                     lane_shift(t.strided, lgtg), 1u << (LG + lgtg), blk, s0, n, cx, !t.strided, last);
 #pragma unroll
     for (int p = 0; p < P; ++p) {
         bool stored = false;
@@ -904,7 +915,8 @@ __device__ __forceinline__ void each_limb(uint64_t limb, uint64_t lstep, const R
 // that the sets' registers do not count against each other.  (Every pass of
 // a call has the same kRelaxOut flag and every kernel that may be launched
 // with it the same modes, so the passes agree on what lies between them.)
-template <bool INV, int LG, int LR, bool CG, bool MUL = false, bool MODES = false, bool RELAX = false, int P = 1>
+template <bool INV, int LG, int LR, bool CG, bool MUL = false, bool MODES = false, bool RELAX = false, int P = 1,
+          int SHAPE = kAnyTiles>
 __device__ __forceinline__ void pass_tile(const uint64_t* src, uint64_t* dst, const ModCtx* cx, uint32_t logn,
                                           uint32_t s0, uint32_t lgtg, uint64_t limb, uint64_t tile_in_limb,
                                           uint32_t flags, uint64_t* sm, const uint64_t* operand = nullptr,
@@ -914,27 +926,27 @@ __device__ __forceinline__ void pass_tile(const uint64_t* src, uint64_t* dst, co
         const uint32_t kind = cx->arith;
         if constexpr (RELAX) {
             if (kind == kFp) {
-                pass_tile_as<kFp, INV, LG, LR, CG, MUL, P>(src, dst, cx, logn, s0, lgtg, limb, lstep, tile_in_limb,
+                pass_tile_as<kFp, INV, LG, LR, CG, MUL, P, SHAPE>(src, dst, cx, logn, s0, lgtg, limb, lstep, tile_in_limb,
                                                            flags, sm, operand);
                 return;
             }
             if (kind == kRelaxed) {
                 each_limb<P>(limb, lstep, [&](uint64_t l) {
-                    pass_tile_as<kRelaxed, INV, LG, LR, CG, MUL, 1>(src, dst, cx, logn, s0, lgtg, l, lstep,
+                    pass_tile_as<kRelaxed, INV, LG, LR, CG, MUL, 1, SHAPE>(src, dst, cx, logn, s0, lgtg, l, lstep,
                                                                        tile_in_limb, flags, sm, operand);
                 });
                 return;
             }
         } else if constexpr (!INV) {
             if (kind == kFp && (flags & kLazyFp)) {
-                pass_tile_as<kFpLazy, INV, LG, LR, CG, MUL, P>(src, dst, cx, logn, s0, lgtg, limb, lstep,
+                pass_tile_as<kFpLazy, INV, LG, LR, CG, MUL, P, SHAPE>(src, dst, cx, logn, s0, lgtg, limb, lstep,
                                                                tile_in_limb, flags, sm, operand);
                 return;
             }
         }
     }
     each_limb<P>(limb, lstep, [&](uint64_t l) {
-        pass_tile_as<kExact, INV, LG, LR, CG, MUL, 1>(src, dst, cx, logn, s0, lgtg, l, lstep, tile_in_limb, flags,
+        pass_tile_as<kExact, INV, LG, LR, CG, MUL, 1, SHAPE>(src, dst, cx, logn, s0, lgtg, l, lstep, tile_in_limb, flags,
                                                          sm, operand);
     });
 }
@@ -955,7 +967,7 @@ __device__ __forceinline__ bool cta_tile(const PassArgs& a, uint32_t lg_tiles, u
     return limb < a.count;
 }
 
-template <bool INV, int LG, int LR, bool RELAX>
+template <bool INV, int LG, int LR, bool RELAX, int SHAPE>
 __global__ void __launch_bounds__(max_threads(LR), LR == 3 ? 2 : 1) ntt_pass_kernel(const __grid_constant__ PassArgs a)
 {
     extern __shared__ uint64_t sm[];
@@ -963,13 +975,13 @@ __global__ void __launch_bounds__(max_threads(LR), LR == 3 ? 2 : 1) ntt_pass_ker
     uint64_t limb, lstep;
     uint32_t til;
     if (!cta_tile<1>(a, a.logn - LG - lgtg, limb, til, lstep)) return;
-    pass_tile<INV, LG, LR, false, false, true, RELAX, 1>(a.src, a.dst, a.ctx[blockIdx.y], a.logn, a.s0, lgtg, limb, til,
+    pass_tile<INV, LG, LR, false, false, true, RELAX, 1, SHAPE>(a.src, a.dst, a.ctx[blockIdx.y], a.logn, a.s0, lgtg, limb, til,
                                                          a.flags, sm, nullptr, lstep);
 }
 
 // Sixteen registers of the limb per thread: held to the machine registers it
 // takes by itself, where four or three CTAs of 256 threads share an SM.
-template <bool INV, int LG>
+template <bool INV, int LG, int SHAPE>
 __global__ void __maxnreg__(INV ? 80 : 72) ntt_pass16_kernel(const __grid_constant__ PassArgs a)
 {
     extern __shared__ uint64_t sm[];
@@ -977,11 +989,11 @@ __global__ void __maxnreg__(INV ? 80 : 72) ntt_pass16_kernel(const __grid_consta
     uint64_t limb, lstep;
     uint32_t til;
     if (!cta_tile<1>(a, a.logn - LG - lgtg, limb, til, lstep)) return;
-    pass_tile<INV, LG, 4, false, false, true, false, 1>(a.src, a.dst, a.ctx[blockIdx.y], a.logn, a.s0, lgtg, limb, til,
+    pass_tile<INV, LG, 4, false, false, true, false, 1, SHAPE>(a.src, a.dst, a.ctx[blockIdx.y], a.logn, a.s0, lgtg, limb, til,
                                                          a.flags, sm, nullptr, lstep);
 }
 
-template <bool INV, int LG, int LR, bool RELAX>
+template <bool INV, int LG, int LR, bool RELAX, int SHAPE>
 __global__ void __maxnreg__(kPairRegs) ntt_pass_pair_kernel(const __grid_constant__ PassArgs a)
 {
     extern __shared__ uint64_t sm[];
@@ -989,14 +1001,14 @@ __global__ void __maxnreg__(kPairRegs) ntt_pass_pair_kernel(const __grid_constan
     uint64_t limb, lstep;
     uint32_t til;
     if (!cta_tile<2>(a, a.logn - LG - lgtg, limb, til, lstep)) return;
-    pass_tile<INV, LG, LR, false, false, true, RELAX, 2>(a.src, a.dst, a.ctx[blockIdx.y], a.logn, a.s0, lgtg, limb, til,
+    pass_tile<INV, LG, LR, false, false, true, RELAX, 2, SHAPE>(a.src, a.dst, a.ctx[blockIdx.y], a.logn, a.s0, lgtg, limb, til,
                                                          a.flags, sm, nullptr, lstep);
 }
 
 // The same pass with the dyadic product of kPreMul / kPostMul: a kernel of
 // its own, so that the product's registers do not count against the plain
 // passes.
-template <bool INV, int LG, int LR, bool RELAX>
+template <bool INV, int LG, int LR, bool RELAX, int SHAPE>
 __global__ void __launch_bounds__(max_threads(LR), LR == 3 ? 2 : 1) ntt_pass_mul_kernel(const __grid_constant__ PassArgs a)
 {
     extern __shared__ uint64_t sm[];
@@ -1004,11 +1016,11 @@ __global__ void __launch_bounds__(max_threads(LR), LR == 3 ? 2 : 1) ntt_pass_mul
     uint64_t limb, lstep;
     uint32_t til;
     if (!cta_tile<1>(a, a.logn - LG - lgtg, limb, til, lstep)) return;
-    pass_tile<INV, LG, LR, false, true, true, RELAX, 1>(a.src, a.dst, a.ctx[blockIdx.y], a.logn, a.s0, lgtg, limb, til,
+    pass_tile<INV, LG, LR, false, true, true, RELAX, 1, SHAPE>(a.src, a.dst, a.ctx[blockIdx.y], a.logn, a.s0, lgtg, limb, til,
                                                         a.flags, sm, a.operand, lstep);
 }
 
-template <bool INV, int LG>
+template <bool INV, int LG, int SHAPE>
 __global__ void __maxnreg__(128) ntt_pass_mul16_kernel(const __grid_constant__ PassArgs a)
 {
     extern __shared__ uint64_t sm[];
@@ -1016,11 +1028,11 @@ __global__ void __maxnreg__(128) ntt_pass_mul16_kernel(const __grid_constant__ P
     uint64_t limb, lstep;
     uint32_t til;
     if (!cta_tile<1>(a, a.logn - LG - lgtg, limb, til, lstep)) return;
-    pass_tile<INV, LG, 4, false, true, true, false, 1>(a.src, a.dst, a.ctx[blockIdx.y], a.logn, a.s0, lgtg, limb, til,
+    pass_tile<INV, LG, 4, false, true, true, false, 1, SHAPE>(a.src, a.dst, a.ctx[blockIdx.y], a.logn, a.s0, lgtg, limb, til,
                                                         a.flags, sm, a.operand, lstep);
 }
 
-template <bool INV, int LG, int LR, bool RELAX>
+template <bool INV, int LG, int LR, bool RELAX, int SHAPE>
 __global__ void __maxnreg__(kPairRegs) ntt_pass_mul_pair_kernel(const __grid_constant__ PassArgs a)
 {
     extern __shared__ uint64_t sm[];
@@ -1028,7 +1040,7 @@ __global__ void __maxnreg__(kPairRegs) ntt_pass_mul_pair_kernel(const __grid_con
     uint64_t limb, lstep;
     uint32_t til;
     if (!cta_tile<2>(a, a.logn - LG - lgtg, limb, til, lstep)) return;
-    pass_tile<INV, LG, LR, false, true, true, RELAX, 2>(a.src, a.dst, a.ctx[blockIdx.y], a.logn, a.s0, lgtg, limb, til,
+    pass_tile<INV, LG, LR, false, true, true, RELAX, 2, SHAPE>(a.src, a.dst, a.ctx[blockIdx.y], a.logn, a.s0, lgtg, limb, til,
                                                         a.flags, sm, a.operand, lstep);
 }
 

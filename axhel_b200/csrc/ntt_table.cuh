@@ -18,7 +18,8 @@ constexpr int kMaxLR = 5;
 // both where relaxed_compiled.
 template <class Fn>
 struct FnTable {
-    Fn at[2][2][kMaxLG + 1][kMaxLR + 1] = {};
+    // Last but two: 0 strided columns, 1 contiguous rows (pass kernels).
+    Fn at[2][2][2][kMaxLG + 1][kMaxLR + 1] = {};
     // Chain and product kernels with the reference's butterflies only, for
     // launches of a few limbs: those run through their code once, and a
     // kernel that holds the other arithmetics too takes 13-20 % longer to
@@ -33,25 +34,38 @@ const FnTable<PassFn>& inv_mul_table();
 const FnTable<ChainFn>& chain_table();
 const FnTable<ChainFn>& product_table();
 
-// Fills a table with Get<LG, LR, RELAX, P>::fn(); P limbs per thread, 0: plain.  Register-stage counts
-// compiled for each group size: LR = LG for tiny groups, otherwise 3, 4 and 5.
-template <template <int, int, bool, int> class Get, class Fn, int LG, int LR>
-void add_one(FnTable<Fn>& t)
+template <template <int, int, bool, int, int> class Get, class Fn, int LG, int LR, int SHAPE>
+void add_shape(FnTable<Fn>& t)
 {
-    if constexpr (LR <= LG && Get<LG, LR, false, 1>::compiled) {
-        t.at[0][0][LG][LR] = Get<LG, LR, false, 1>::fn();
-        t.plain[LG][LR] = t.at[0][0][LG][LR];
-        if constexpr (relaxed_compiled(LG, LR) && Get<LG, LR, false, 1>::has_plain)
-            t.plain[LG][LR] = Get<LG, LR, false, 0>::fn();
-        if constexpr (relaxed_compiled(LG, LR)) {
-            t.at[1][0][LG][LR] = Get<LG, LR, true, 1>::fn();
-            t.at[0][1][LG][LR] = Get<LG, LR, false, 2>::fn();
-            t.at[1][1][LG][LR] = Get<LG, LR, true, 2>::fn();
-        }
+    constexpr int row = SHAPE == kRowTiles;
+    t.at[0][0][row][LG][LR] = Get<LG, LR, false, 1, SHAPE>::fn();
+    if constexpr (relaxed_compiled(LG, LR)) {
+        t.at[1][0][row][LG][LR] = Get<LG, LR, true, 1, SHAPE>::fn();
+        t.at[0][1][row][LG][LR] = Get<LG, LR, false, 2, SHAPE>::fn();
+        t.at[1][1][row][LG][LR] = Get<LG, LR, true, 2, SHAPE>::fn();
     }
 }
 
-template <template <int, int, bool, int> class Get, class Fn, int... I>
+// Fills a table with Get<LG, LR, RELAX, P, SHAPE>::fn(); P limbs per thread, 0: plain.  Register-stage counts
+// compiled for each group size: LR = LG for tiny groups, otherwise 3, 4 and 5.
+template <template <int, int, bool, int, int> class Get, class Fn, int LG, int LR>
+void add_one(FnTable<Fn>& t)
+{
+    if constexpr (LR <= LG && Get<LG, LR, false, 1, kRowTiles>::compiled) {
+        add_shape<Get, Fn, LG, LR, kRowTiles>(t);
+        if constexpr (Get<LG, LR, false, 1, kRowTiles>::shaped) {
+            add_shape<Get, Fn, LG, LR, kColumnTiles>(t);
+        } else {
+            for (auto& relax : t.at)
+                for (auto& pair : relax) pair[0][LG][LR] = pair[1][LG][LR];
+        }
+        t.plain[LG][LR] = t.at[0][0][1][LG][LR];
+        if constexpr (relaxed_compiled(LG, LR) && Get<LG, LR, false, 1, kRowTiles>::has_plain)
+            t.plain[LG][LR] = Get<LG, LR, false, 0, kRowTiles>::fn();
+    }
+}
+
+template <template <int, int, bool, int, int> class Get, class Fn, int... I>
 FnTable<Fn> make_table(std::integer_sequence<int, I...>)
 {
     FnTable<Fn> t;
