@@ -94,9 +94,26 @@ def build_tools(force=False):
             raise RuntimeError(f"tool build failed: {' '.join(cmd)}\n{r.stdout}\n{r.stderr}")
 
 
+def build_pyext(force=False):
+    """The Python extension ``axhel_b200/_fastcall.so`` (pyext/fastcall.c)."""
+    import sysconfig
+
+    src = os.path.join(PKG, "pyext", "fastcall.c")
+    out = os.path.join(PKG, "_fastcall.so")
+    if not force and os.path.exists(out) and os.path.getmtime(out) >= os.path.getmtime(src):
+        return
+    cmd = ["gcc", "-O2", "-Wall", "-Wextra", "-shared", "-fPIC", "-I" + sysconfig.get_paths()["include"], src, "-o",
+           out + ".tmp"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"extension build failed: {' '.join(cmd)}\n{r.stdout}\n{r.stderr}")
+    os.replace(out + ".tmp", out)
+
+
 def build(force=False, verbose_ptxas=False, quiet=False):
-    """Compile and link libaxhel.so (and the tools); returns its path."""
+    """Compile and link libaxhel.so (and the extension and the tools); returns its path."""
     lib = _build_lib(force, verbose_ptxas, quiet)
+    build_pyext(force)
     build_tools(force)
     return lib
 

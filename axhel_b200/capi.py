@@ -10,6 +10,11 @@ from __future__ import annotations
 import ctypes as C
 import os
 
+try:
+    from ._fastcall import call as _fast
+except ImportError as e:
+    raise RuntimeError("axhel_b200/_fastcall.so not built (run python -m axhel_b200.build)") from e
+
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "libaxhel.so")
 
@@ -96,8 +101,45 @@ def lib():
             raise RuntimeError(f"AXHEL CUDA library not built: {LIB_PATH} (run python -m axhel_b200.build)")
         L = C.CDLL(LIB_PATH)
         _declare(L)
+        for name in _HOT:
+            _hot[name] = C.cast(getattr(L, "axhel_cuda_" + name), vp).value
         _lib = L
     return _lib
+
+
+# The entry points called per limb or batch go through the extension: their
+# argument conversions through ctypes cost as much as half a launch.
+_HOT = ("ntt_forward", "ntt_inverse", "ntt_forward_batch", "ntt_inverse_batch", "ntt_chain_mul_batch",
+        "ntt_chain_fma_batch", "ntt_product_batch", "ntt_forward_mul_batch", "ntt_mul_inverse_batch",
+        "eltwise_add_vv", "eltwise_add_vs", "eltwise_sub_vv", "eltwise_sub_vs", "eltwise_mul", "eltwise_fma",
+        "eltwise_reduce", "tensor_product")
+
+
+class _Hot(dict):
+    """Addresses of the hot entry points; the first lookup loads the library."""
+
+    def __missing__(self, name):
+        lib()
+        return self[name]
+
+
+_hot = _Hot()
+
+
+def _call(name, where, *args):
+    try:
+        st = _fast(_hot[name], *args)
+    except TypeError:
+        # an address given as a ctypes object: ctypes' own conversions
+        st = getattr(lib(), "axhel_cuda_" + name)(*[_array(a) if isinstance(a, (list, tuple)) else a for a in args])
+    if st:
+        check(st, where)
+
+
+def _array(items):
+    if items and not isinstance(items[0], int):
+        return (vp * len(items))(*[t.h.value for t in items])
+    return C.cast((u64 * len(items))(*items), vp)
 
 
 def _declare(L):
@@ -374,11 +416,6 @@ class Server:
             pass
 
 
-def _arr64(values):
-    a = (u64 * len(values))(*[int(v) for v in values])
-    return a
-
-
 class NTT:
     """A device-resident (N, q) table context (``axhel_ntt_t``)."""
 
@@ -395,6 +432,7 @@ class NTT:
             check(lib().axhel_cuda_ntt_create_external(degree, modulus, fwd.ctypes.data, inv.ctypes.data,
                                                        ninv.ctypes.data, C.byref(h)), "ntt_create_external")
         self.h = h
+        self.hv = h.value or 0  # the handle as an int, for the extension
         self.degree = degree
         self.modulus = modulus
 
@@ -413,6 +451,7 @@ class NTT:
         if self.h:
             lib().axhel_cuda_ntt_release(self.h)
             self.h = vp()
+            self.hv = 0
 
     def __del__(self):
         try:
@@ -431,82 +470,75 @@ class NTT:
         return fwd, inv, ninv
 
     def forward(self, dst, src, in_f=1, out_f=1, stream=0):
-        check(lib().axhel_cuda_ntt_forward(self.h, dst, src, in_f, out_f, stream), "ntt_forward")
+        _call("ntt_forward", "ntt_forward", self.hv, dst, src, in_f, out_f, stream)
 
     def inverse(self, dst, src, in_f=1, out_f=1, stream=0):
-        check(lib().axhel_cuda_ntt_inverse(self.h, dst, src, in_f, out_f, stream), "ntt_inverse")
+        _call("ntt_inverse", "ntt_inverse", self.hv, dst, src, in_f, out_f, stream)
 
 
-def _handles(ntts):
-    return (vp * len(ntts))(*[t.h.value for t in ntts])
+def _seq(ntts):
+    return ntts if isinstance(ntts, (list, tuple)) else list(ntts)
 
 
 def forward_batch(ntts, dst, src, count, in_f=1, out_f=1, stream=0):
-    check(lib().axhel_cuda_ntt_forward_batch(_handles(ntts), len(ntts), dst, src, count, in_f, out_f, stream),
-          "ntt_forward_batch")
+    _call("ntt_forward_batch", "ntt_forward_batch", _seq(ntts), len(ntts), dst, src, count, in_f, out_f, stream)
 
 
 def inverse_batch(ntts, dst, src, count, in_f=1, out_f=1, stream=0):
-    check(lib().axhel_cuda_ntt_inverse_batch(_handles(ntts), len(ntts), dst, src, count, in_f, out_f, stream),
-          "ntt_inverse_batch")
+    _call("ntt_inverse_batch", "ntt_inverse_batch", _seq(ntts), len(ntts), dst, src, count, in_f, out_f, stream)
 
 
 def forward_mul_batch(ntts, dst, src, multiplicand, count, stream=0):
     """Forward transform of each limb, then the dyadic product with `multiplicand`."""
-    check(lib().axhel_cuda_ntt_forward_mul_batch(_handles(ntts), len(ntts), dst, src, multiplicand, count, stream),
-          "ntt_forward_mul_batch")
+    _call("ntt_forward_mul_batch", "ntt_forward_mul_batch", _seq(ntts), len(ntts), dst, src, multiplicand, count,
+          stream)
 
 
 def mul_inverse_batch(ntts, dst, src, multiplicand, count, out_f=1, stream=0):
     """Dyadic product with `multiplicand`, then the inverse transform of each limb."""
-    check(lib().axhel_cuda_ntt_mul_inverse_batch(_handles(ntts), len(ntts), dst, src, multiplicand, count, out_f,
-                                                 stream), "ntt_mul_inverse_batch")
+    _call("ntt_mul_inverse_batch", "ntt_mul_inverse_batch", _seq(ntts), len(ntts), dst, src, multiplicand, count,
+          out_f, stream)
 
 
 def chain_mul_batch(ntts, dst, src, multiplicand, count, in_f=2, out_f=1, stream=0):
-    check(lib().axhel_cuda_ntt_chain_mul_batch(_handles(ntts), len(ntts), dst, src, multiplicand, count, in_f, out_f,
-                                               stream), "ntt_chain_mul_batch")
+    _call("ntt_chain_mul_batch", "ntt_chain_mul_batch", _seq(ntts), len(ntts), dst, src, multiplicand, count, in_f,
+          out_f, stream)
 
 
 def product_batch(ntts, dst, src, multiplicand, count, in_f=4, out_f=1, stream=0):
     """Fused NTT -> MulMod(., multiplicand, 4) -> INTT over a batch."""
-    hs = _handles(ntts)
-    check(lib().axhel_cuda_ntt_product_batch(hs, len(ntts), dst, src, multiplicand, count, in_f, out_f, stream),
-          "ntt_product_batch")
+    _call("ntt_product_batch", "ntt_product_batch", _seq(ntts), len(ntts), dst, src, multiplicand, count, in_f, out_f,
+          stream)
 
 
 def chain_fma_batch(ntts, dst, src, scalars, addend, count, in_f=2, out_f=1, stream=0):
-    sc = _arr64(scalars)
-    check(lib().axhel_cuda_ntt_chain_fma_batch(_handles(ntts), len(ntts), dst, src, C.cast(sc, vp), addend, count,
-                                               in_f, out_f, stream), "ntt_chain_fma_batch")
+    _call("ntt_chain_fma_batch", "ntt_chain_fma_batch", _seq(ntts), len(ntts), dst, src, [int(v) for v in scalars],
+          addend, count, in_f, out_f, stream)
 
 
 def add(dst, a, b, n, q, stream=0, scalar=False):
-    f = lib().axhel_cuda_eltwise_add_vs if scalar else lib().axhel_cuda_eltwise_add_vv
-    check(f(dst, a, b, n, q, stream), "eltwise_add")
+    _call("eltwise_add_vs" if scalar else "eltwise_add_vv", "eltwise_add", dst, a, b, n, q, stream)
 
 
 def sub(dst, a, b, n, q, stream=0, scalar=False):
-    f = lib().axhel_cuda_eltwise_sub_vs if scalar else lib().axhel_cuda_eltwise_sub_vv
-    check(f(dst, a, b, n, q, stream), "eltwise_sub")
+    _call("eltwise_sub_vs" if scalar else "eltwise_sub_vv", "eltwise_sub", dst, a, b, n, q, stream)
 
 
 def mul(dst, a, b, n, q, factor, stream=0):
-    check(lib().axhel_cuda_eltwise_mul(dst, a, b, n, q, factor, stream), "eltwise_mul")
+    _call("eltwise_mul", "eltwise_mul", dst, a, b, n, q, factor, stream)
 
 
 def fma(dst, a, s, c, n, q, factor, stream=0):
-    check(lib().axhel_cuda_eltwise_fma(dst, a, s, c, n, q, factor, stream), "eltwise_fma")
+    _call("eltwise_fma", "eltwise_fma", dst, a, s, c, n, q, factor, stream)
 
 
 def reduce(dst, a, n, q, in_f, out_f, stream=0):
-    check(lib().axhel_cuda_eltwise_reduce(dst, a, n, q, in_f, out_f, stream), "eltwise_reduce")
+    _call("eltwise_reduce", "eltwise_reduce", dst, a, n, q, in_f, out_f, stream)
 
 
 def tensor_product(r0, r1, r2, c0, c1, d0, d1, n, count, moduli, factor=1, stream=0):
-    m = _arr64(moduli)
-    check(lib().axhel_cuda_tensor_product(r0, r1, r2, c0, c1, d0, d1, n, count, C.cast(m, vp), len(moduli), factor,
-                                          stream), "tensor_product")
+    m = [int(v) for v in moduli]
+    _call("tensor_product", "tensor_product", r0, r1, r2, c0, c1, d0, d1, n, count, m, len(m), factor, stream)
 
 
 def plan_set(inverse, logn, passes):
