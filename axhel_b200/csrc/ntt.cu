@@ -101,6 +101,12 @@ bool plan_relax(NttPlan& p)
     NttPlan r = p;
     for (int i = 0; i < p.npass; ++i) {
         PassCfg& c = r.pass[i];
+        // A pass tuned with 16 registers per thread takes twice the threads
+        // here; back to 128 where the tile keeps 8 columns (64-byte rows).
+        // The 7-stage passes of 768 limbs of N = 2^16, 16 against 8 columns:
+        // 242 to 224 us forward, 285 to 264 inverse (4 columns at 8 stages
+        // or 8 at 6: 3-10 % slower).
+        if (c.lr == 4 && (c.tg << (c.lg - 3)) > 128 && c.tg > 8) c.tg >>= 1;
         c.lr = 3;
         if (!pass_relaxable(c) || ((uint64_t)c.tg << (c.lg - c.lr)) > (uint64_t)max_threads(c.lr)) return false;
     }
