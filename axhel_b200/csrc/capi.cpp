@@ -460,19 +460,18 @@ bool fp_any(const axhel_ntt_t* ntts, uint64_t n_ntts) { return fp_moduli(ntts, n
 // Whether a quarter of the moduli or more have FP64 forms.
 bool fp_share(const axhel_ntt_t* ntts, uint64_t n_ntts) { return 4 * fp_moduli(ntts, n_ntts) >= n_ntts; }
 
-// Few enough limbs for the cluster form, whose kernels hold the reference's
-// butterflies only, but the passes in FP64 are faster: from 2^17 residues on
-// (64 limbs of N = 2^12: forward 5.5 against 5.7 us, chain 8.8 against 10.0;
-// 16 of 2^13 5.2 against 5.4, of 2^14 6.0 against 7.8) and from N = 2^15 on
-// (one limb 5.2 against 7.3, chain 9.6 against 12.3; at 2^14 4.9 against 4.5
-// and 9.2 against 8.3).
-// For the fused chains below N = 2^14 the line is twice that (16 limbs of 2^13
-// 9.3 against 8.7 us), likewise where the forward is lazy (8 of 2^14: 12.0
-// against 10.8; 16: 12.6 against 15.0).
-bool fp_passes_win(const axhel_ntt_t* ntts, uint64_t n_ntts, uint32_t logn, uint64_t count, bool fused, bool lazy)
+// Few enough limbs for the one-launch cluster form of a fused chain or product,
+// whose kernels hold the reference's butterflies only, but three passes in
+// FP64 are faster although they cost two launches more: from 2^18 residues on.
+// Calls one after the other, us, cluster form then passes: 66 limbs of
+// N = 2^12 18.8 and 10.5, 6 limbs of 2^15 22.8 and 16.5; below that line 4
+// limbs of 2^15 14.5 and 14.9 (lazy chain 14.5 and 18.6).  Not for single
+// transforms: one limb of 2^15 takes 5.2 us as two passes against 7.3 on the
+// device, but calls one after the other are bound by the second launch (8
+// limbs of 2^14 8.3 and 10.4).
+bool fp_passes_win(const axhel_ntt_t* ntts, uint64_t n_ntts, uint32_t logn, uint64_t count)
 {
-    const uint64_t words = (fused && logn < 14) || lazy ? 1ull << 18 : 1ull << 17;
-    return ((count << logn) >= words || logn >= 15) && fp_moduli(ntts, n_ntts) == n_ntts;
+    return (count << logn) >= (1ull << 18) && fp_moduli(ntts, n_ntts) == n_ntts;
 }
 
 // Runs the passes of `plan` in order; pass i reads `src` (first pass) or
@@ -539,8 +538,7 @@ axhel_status_t transform(bool inverse, const axhel_ntt_t* ntts, uint64_t n_ntts,
     ClusterCfg cc;
     const bool norm = ((first | last) & (kPostNorm | kPostMul)) != 0;
     if (!plan_overridden(inverse, a.logn) &&
-        cluster_plan(inverse ? kClusterInverse : kClusterForward, a.logn, count, &cc) &&
-        !(norm && fp_passes_win(ntts, n_ntts, a.logn, count, false, false))) {
+        cluster_plan(inverse ? kClusterInverse : kClusterForward, a.logn, count, &cc)) {
         a.src = operand;
         a.dst = result;
         a.s0 = 0;
@@ -578,7 +576,7 @@ axhel_status_t chain(const axhel_ntt_t* ntts, uint64_t n_ntts, uint64_t* result,
     // a few limbs: the whole chain in one launch, one cluster per limb
     ClusterCfg cc;
     if (!plan_overridden(true, logn) && cluster_plan(kClusterChain, logn, count, &cc) &&
-        !fp_passes_win(ntts, n_ntts, logn, count, true, out_f == 4)) {
+        !fp_passes_win(ntts, n_ntts, logn, count)) {
         c.pass.src = operand;
         c.pass.dst = result;
         c.pass.flags = (in_f == 4 ? (uint32_t)kPreCsub2q : 0u) | (out_f != 4 ? (uint32_t)kPostNorm : 0u);
@@ -673,7 +671,7 @@ axhel_status_t product(const axhel_ntt_t* ntts, uint64_t n_ntts, uint64_t* resul
     // a few limbs: the whole product in one launch, one cluster per limb
     ClusterCfg cc;
     if (!plan_overridden(true, logn) && cluster_plan(kClusterProduct, logn, count, &cc) &&
-        !fp_passes_win(ntts, n_ntts, logn, count, true, out_f == 2)) {
+        !fp_passes_win(ntts, n_ntts, logn, count)) {
         c.pass.src = operand;
         c.pass.dst = result;
         c.pass.flags = out_f != 2 ? (uint32_t)kPostNorm : 0u;
