@@ -34,7 +34,7 @@
 // LG = 5..9 of the degrees 2^10 .. 2^17 (a tile never spans two limbs or two
 // blocks), handled by 128 threads x 8 registers (LR = 3) in the persistent
 // kernel.  The per-phase launches run one kernel per tile class and pass
-// width (64 threads x 16 registers for the 7-stage transform passes), each
+// width (64 threads x 16 registers for the 7-stage passes of exact butterflies), each
 // phase's largest entries in launches of their own that take the entry as a
 // kernel parameter, side by side on extra streams.
 // The same tile functions as the plain kernels run the butterflies

@@ -1,8 +1,8 @@
 // Device-side modular arithmetic on 64-bit residues (q < 2^62).
 //
-// Every routine reproduces, operation for operation, the reference native
-// backend's formula it names, so results are bit-identical including the lazy
-// representatives in [0, 2q) / [0, 4q).  64x64->128 products use
+// The routines that name a formula of the reference's native backend
+// reproduce it operation for operation, so results are bit-identical including
+// the lazy representatives in [0, 2q) / [0, 4q).  64x64->128 products use
 // __umul64hi / 64-bit mul.lo, no tensor cores.  Where only the residue
 // matters (intermediate values of a transform whose output is reduced to
 // [0, q)), the relaxed and FP64 forms below compute the same residues with

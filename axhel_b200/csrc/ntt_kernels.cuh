@@ -18,13 +18,15 @@
 // with one barrier per exchange.  Global accesses are coalesced: in strided
 // tiles consecutive lanes take consecutive columns; in contiguous tiles a
 // round whose register bits are the low bits reads R consecutive words per
-// thread as 16-byte vectors, and the other rounds read runs of 2^lo words.
+// thread as 32- or 16-byte vectors, and the other rounds read runs of 2^lo words.
 //
-// Every butterfly is exactly the reference's (ForwardButterflyNative /
+// The butterflies are the reference's (ForwardButterflyNative /
 // InverseButterflyNative, axhel/ntt/ntt-internal.hpp:20-49, and the final
-// inverse stage of axhel/ntt/ntt-native.cpp:126-141), applied to the same
-// element pairs with the same twiddles in the same stage order, so outputs
-// are bit-identical, lazy ranges included.  Twiddle indices:
+// inverse stage of axhel/ntt/ntt-native.cpp:126-141) on the same element
+// pairs with the same twiddles in the same stage order: operation for
+// operation where the output is lazy, on other representatives of the same
+// residues where it is canonical (the modes below), so outputs are
+// bit-identical, lazy ranges included.  Twiddle indices:
 //   forward stage t, position p : fwd[2^t + (p >> (logn - t))]      (ntt-native.cpp:39)
 //   inverse stage s, position p : inv[1 + N - N/2^s + (p >> (s+1))]  (ntt-native.cpp:84, the
 //                                 sequential root_index over the blocks of each stage)
