@@ -11,7 +11,7 @@ import ctypes as C
 import os
 
 try:
-    from ._fastcall import call as _fast
+    from ._fastcall import call as _fast, handle_type as _handle_type
 except ImportError as e:
     raise RuntimeError("axhel_b200/_fastcall.so not built (run python -m axhel_b200.build)") from e
 
@@ -108,11 +108,32 @@ def lib():
 
 
 # The entry points called per limb or batch go through the extension: their
-# argument conversions through ctypes cost as much as half a launch.
-_HOT = ("ntt_forward", "ntt_inverse", "ntt_forward_batch", "ntt_inverse_batch", "ntt_chain_mul_batch",
-        "ntt_chain_fma_batch", "ntt_product_batch", "ntt_forward_mul_batch", "ntt_mul_inverse_batch",
-        "eltwise_add_vv", "eltwise_add_vs", "eltwise_sub_vv", "eltwise_sub_vs", "eltwise_mul", "eltwise_fma",
-        "eltwise_reduce", "tensor_product")
+# argument conversions through ctypes cost as much as half a launch.  One
+# letter per argument: i an integer, p an address, h a list of NTT objects and
+# a one of integers, as arrays.
+_HOT = {
+    "ntt_forward": "pppiip",
+    "ntt_inverse": "pppiip",
+    "ntt_forward_batch": "hippiiip",
+    "ntt_inverse_batch": "hippiiip",
+    "ntt_chain_mul_batch": "hipppiiip",
+    "ntt_chain_fma_batch": "hippapiiip",
+    "ntt_product_batch": "hipppiiip",
+    "ntt_forward_mul_batch": "hipppip",
+    "ntt_mul_inverse_batch": "hipppiip",
+    "eltwise_add_vv": "pppiip",
+    "eltwise_add_vs": "ppiiip",
+    "eltwise_sub_vv": "pppiip",
+    "eltwise_sub_vs": "ppiiip",
+    "eltwise_mul": "pppiiip",
+    "eltwise_fma": "ppipiiip",
+    "eltwise_reduce": "ppiiiip",
+    "tensor_product": "pppppppiiaiip",
+}
+
+
+_ARRAYS = {"h": lambda ntts: (vp * len(ntts))(*[t.h.value for t in ntts]),
+           "a": lambda values: C.cast((u64 * len(values))(*values), vp)}
 
 
 class _Hot(dict):
@@ -127,19 +148,13 @@ _hot = _Hot()
 
 
 def _call(name, where, *args):
-    try:
-        st = _fast(_hot[name], *args)
-    except TypeError:
-        # an address given as a ctypes object: ctypes' own conversions
-        st = getattr(lib(), "axhel_cuda_" + name)(*[_array(a) if isinstance(a, (list, tuple)) else a for a in args])
+    st = _fast(_hot[name], _HOT[name], *args)
+    if st is None:
+        # an argument in another form than the extension's: ctypes converts or refuses it
+        args = [_ARRAYS[k](x) if k in _ARRAYS else x for k, x in zip(_HOT[name], args)]
+        st = getattr(lib(), "axhel_cuda_" + name)(*args)
     if st:
         check(st, where)
-
-
-def _array(items):
-    if items and not isinstance(items[0], int):
-        return (vp * len(items))(*[t.h.value for t in items])
-    return C.cast((u64 * len(items))(*items), vp)
 
 
 def _declare(L):
@@ -476,8 +491,15 @@ class NTT:
         _call("ntt_inverse", "ntt_inverse", self.hv, dst, src, in_f, out_f, stream)
 
 
+_handle_type(NTT)
+
+
 def _seq(ntts):
-    return ntts if isinstance(ntts, (list, tuple)) else list(ntts)
+    return ntts if isinstance(ntts, (list, tuple)) else list(ntts) if len(ntts) else []
+
+
+def _ints(values):
+    return [int(v) for v in values] if len(values) else []
 
 
 def forward_batch(ntts, dst, src, count, in_f=1, out_f=1, stream=0):
@@ -512,8 +534,8 @@ def product_batch(ntts, dst, src, multiplicand, count, in_f=4, out_f=1, stream=0
 
 
 def chain_fma_batch(ntts, dst, src, scalars, addend, count, in_f=2, out_f=1, stream=0):
-    _call("ntt_chain_fma_batch", "ntt_chain_fma_batch", _seq(ntts), len(ntts), dst, src, [int(v) for v in scalars],
-          addend, count, in_f, out_f, stream)
+    _call("ntt_chain_fma_batch", "ntt_chain_fma_batch", _seq(ntts), len(ntts), dst, src, _ints(scalars), addend,
+          count, in_f, out_f, stream)
 
 
 def add(dst, a, b, n, q, stream=0, scalar=False):
@@ -537,7 +559,7 @@ def reduce(dst, a, n, q, in_f, out_f, stream=0):
 
 
 def tensor_product(r0, r1, r2, c0, c1, d0, d1, n, count, moduli, factor=1, stream=0):
-    m = [int(v) for v in moduli]
+    m = _ints(moduli)
     _call("tensor_product", "tensor_product", r0, r1, r2, c0, c1, d0, d1, n, count, m, len(m), factor, stream)
 
 

@@ -5,6 +5,10 @@
 // launches behind it: a third of a small transform's host time.  call() passes
 // up to 14 integers (System V: every argument of these functions is an
 // integer or pointer of at most 64 bits in a register or 8-byte stack slot).
+//
+// It converts the plain argument forms only, each as ctypes converts it, and
+// answers None without a call for any other, which capi.py then gives to
+// ctypes: what is taken and what is refused is ctypes' decision.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 #include <stdint.h>
@@ -15,85 +19,141 @@
 typedef int32_t (*fn_t)(uint64_t, uint64_t, uint64_t, uint64_t, uint64_t, uint64_t, uint64_t, uint64_t, uint64_t,
                         uint64_t, uint64_t, uint64_t, uint64_t, uint64_t);
 
-static PyObject* s_hv;  // attribute of NTT: its handle's address as an int
+static PyObject* s_hv;      // attribute of NTT: its handle's address as an int
+static PyObject* ntt_type;  // capi.NTT
 
-static int as_u64(PyObject* o, uint64_t* out)
+// 1: converted, 0: another form, -1: error.
+static int from_int(PyObject* o, uint64_t* out)
 {
-    if (o == Py_None) {
-        *out = 0;
-        return 0;
-    }
-    if (!PyLong_Check(o)) {
-        PyErr_Format(PyExc_TypeError, "expected an integer, got %.100s", Py_TYPE(o)->tp_name);
-        return -1;
-    }
+    if (!PyLong_Check(o)) return 0;
     *out = PyLong_AsUnsignedLongLongMask(o);
-    return *out == (uint64_t)-1 && PyErr_Occurred() ? -1 : 0;
+    return *out == (uint64_t)-1 && PyErr_Occurred() ? -1 : 1;
 }
 
-// call(address, *args) -> status.  An argument is an int, None (0), or a list
-// or tuple of ints or of NTT objects, passed as the address of an array of
-// their values, with an element count the caller passes itself.
+// An integer parameter: anything with __index__, as for a c_uint64.
+static int from_index(PyObject* o, uint64_t* out)
+{
+    if (PyLong_Check(o)) return from_int(o, out);
+    if (!PyIndex_Check(o)) return 0;
+    PyObject* v = PyNumber_Index(o);
+    if (!v) {
+        PyErr_Clear();
+        return 0;
+    }
+    const int r = from_int(v, out);
+    Py_DECREF(v);
+    return r;
+}
+
+// An address: an int, or None for null, as for a c_void_p.
+static int from_address(PyObject* o, uint64_t* out)
+{
+    if (o != Py_None) return from_int(o, out);
+    *out = 0;
+    return 1;
+}
+
+// The address of an NTT object's handle.
+static int from_ntt(PyObject* o, uint64_t* out)
+{
+    if (!ntt_type || !PyObject_TypeCheck(o, (PyTypeObject*)ntt_type)) return 0;
+    PyObject* v = PyObject_GetAttr(o, s_hv);
+    if (!v) {
+        PyErr_Clear();
+        return 0;
+    }
+    const int r = from_int(v, out);
+    Py_DECREF(v);
+    return r;
+}
+
+// call(address, kinds, *args) -> status, or None if an argument has another
+// form.  kinds: one letter per argument, "i" an integer, "p" an address, "h" a
+// list or tuple of NTT objects and "a" one of ints, these two passed as the
+// address of an array of their values (the caller passes their count too).
 static PyObject* call(PyObject* self, PyObject* const* args, Py_ssize_t nargs)
 {
     (void)self;
     uint64_t a[MAX_ARGS] = {0}, items[MAX_ITEMS], addr;
     uint64_t* heap[MAX_ARGS] = {0};
-    Py_ssize_t used = 0;
-    PyObject* ret = NULL;
-    if (nargs < 1 || nargs > MAX_ARGS + 1) {
-        PyErr_SetString(PyExc_TypeError, "call(address, up to 14 arguments)");
+    Py_ssize_t used = 0, len = 0;
+    const char* kinds = nargs >= 2 && PyUnicode_Check(args[1]) ? PyUnicode_AsUTF8AndSize(args[1], &len) : NULL;
+    if (!kinds || len > MAX_ARGS || nargs != len + 2 || from_int(args[0], &addr) != 1) {
+        if (!PyErr_Occurred()) PyErr_SetString(PyExc_TypeError, "call(address, kinds, one argument per kind)");
         return NULL;
     }
-    if (as_u64(args[0], &addr)) return NULL;
-    for (Py_ssize_t i = 1; i < nargs; ++i) {
-        PyObject* o = args[i];
-        if (!PyList_Check(o) && !PyTuple_Check(o)) {
-            if (as_u64(o, &a[i - 1])) goto done;
+    int r = 1;
+    for (Py_ssize_t i = 0; r == 1 && i < len; ++i) {
+        PyObject* o = args[i + 2];
+        const char kind = kinds[i];
+        if (kind == 'i') {
+            r = from_index(o, &a[i]);
             continue;
+        }
+        if (kind == 'p') {
+            r = from_address(o, &a[i]);
+            continue;
+        }
+        if (!PyList_Check(o) && !PyTuple_Check(o)) {
+            r = 0;
+            break;
         }
         const Py_ssize_t n = PySequence_Fast_GET_SIZE(o);
         uint64_t* to = items + used;
         if (n > MAX_ITEMS - used) {
-            to = heap[i - 1] = PyMem_Malloc((size_t)n * sizeof(uint64_t));
+            to = heap[i] = PyMem_Malloc((size_t)n * sizeof(uint64_t));
             if (!to) {
                 PyErr_NoMemory();
-                goto done;
+                r = -1;
+                break;
             }
         } else {
             used += n;
         }
-        for (Py_ssize_t k = 0; k < n; ++k) {
-            if (k >= PySequence_Fast_GET_SIZE(o)) {  // an attribute lookup below may run Python code
+        for (Py_ssize_t k = 0; r == 1 && k < n; ++k) {
+            if (k >= PySequence_Fast_GET_SIZE(o)) {  // an attribute lookup may run Python code
                 PyErr_SetString(PyExc_RuntimeError, "list changed during the call");
-                goto done;
+                r = -1;
+                break;
             }
             PyObject* e = PySequence_Fast_GET_ITEM(o, k);
-            if (PyLong_Check(e) || e == Py_None) {
-                if (as_u64(e, &to[k])) goto done;
-            } else {
-                PyObject* v = PyObject_GetAttr(e, s_hv);
-                if (!v) goto done;
-                const int bad = as_u64(v, &to[k]);
-                Py_DECREF(v);
-                if (bad) goto done;
-            }
+            Py_INCREF(e);
+            r = kind == 'h' ? from_ntt(e, &to[k]) : from_int(e, &to[k]);
+            Py_DECREF(e);
         }
-        a[i - 1] = (uint64_t)(uintptr_t)to;
+        a[i] = (uint64_t)(uintptr_t)to;
     }
-    int32_t st;
-    Py_BEGIN_ALLOW_THREADS
-    st = ((fn_t)(uintptr_t)addr)(a[0], a[1], a[2], a[3], a[4], a[5], a[6], a[7], a[8], a[9], a[10], a[11], a[12],
-                                 a[13]);
-    Py_END_ALLOW_THREADS
-    ret = PyLong_FromLong(st);
-done:
+    PyObject* ret = NULL;
+    if (r == 1) {
+        int32_t st;
+        Py_BEGIN_ALLOW_THREADS
+        st = ((fn_t)(uintptr_t)addr)(a[0], a[1], a[2], a[3], a[4], a[5], a[6], a[7], a[8], a[9], a[10], a[11], a[12],
+                                     a[13]);
+        Py_END_ALLOW_THREADS
+        ret = PyLong_FromLong(st);
+    } else if (r == 0) {
+        ret = Py_NewRef(Py_None);
+    }
     for (int i = 0; i < MAX_ARGS; ++i) PyMem_Free(heap[i]);
     return ret;
 }
 
-static PyMethodDef methods[] = {{"call", (PyCFunction)(void (*)(void))call, METH_FASTCALL, "call(address, *args) -> status"},
-                                {NULL, NULL, 0, NULL}};
+// handle_type(cls): the class whose objects an "h" list holds.
+static PyObject* handle_type(PyObject* self, PyObject* cls)
+{
+    (void)self;
+    if (!PyType_Check(cls)) {
+        PyErr_SetString(PyExc_TypeError, "expected a class");
+        return NULL;
+    }
+    Py_XSETREF(ntt_type, Py_NewRef(cls));
+    Py_RETURN_NONE;
+}
+
+static PyMethodDef methods[] = {
+    {"call", (PyCFunction)(void (*)(void))call, METH_FASTCALL, "call(address, kinds, *args) -> status or None"},
+    {"handle_type", handle_type, METH_O, "handle_type(cls)"},
+    {NULL, NULL, 0, NULL}};
 static struct PyModuleDef module = {PyModuleDef_HEAD_INIT, "_fastcall", NULL, -1, methods, NULL, NULL, NULL, NULL};
 
 PyMODINIT_FUNC PyInit__fastcall(void)
