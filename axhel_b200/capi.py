@@ -447,9 +447,17 @@ class NTT:
             check(lib().axhel_cuda_ntt_create_external(degree, modulus, fwd.ctypes.data, inv.ctypes.data,
                                                        ninv.ctypes.data, C.byref(h)), "ntt_create_external")
         self.h = h
-        self.hv = h.value or 0  # the handle as an int, for the extension
         self.degree = degree
         self.modulus = modulus
+
+    @property
+    def h(self):
+        return self._h
+
+    @h.setter
+    def h(self, handle):
+        self._h = handle
+        self.hv = handle.value or 0  # as an int, for the extension
 
     @staticmethod
     def create_many(params):
@@ -466,7 +474,6 @@ class NTT:
         if self.h:
             lib().axhel_cuda_ntt_release(self.h)
             self.h = vp()
-            self.hv = 0
 
     def __del__(self):
         try:

@@ -18,7 +18,6 @@ def fake(address=64):
     """An NTT whose handle is never read: the calls below are refused before."""
     t = capi.NTT.__new__(capi.NTT)
     t.h = C.c_void_p(address)
-    t.hv = address
     t.close = lambda: None  # __del__ must not release it
     return t
 
@@ -94,3 +93,16 @@ def test_closed_handle_is_refused():
         with pytest.raises(capi.AxhelError) as e:
             call()
         assert e.value.status == 1
+
+
+def test_replaced_handle_is_the_one_passed():
+    """In a process of its own: a handle kept from before would be read."""
+    code = ("import ctypes as C\n"
+            "from axhel_b200 import capi\n"
+            "t = capi.NTT(8, 17, handle=C.c_void_p(64))\n"
+            "t.h = C.c_void_p(0)\n"
+            "for call in (lambda: t.forward(8, 8), lambda: capi.forward_batch([t], 8, 8, 1)):\n"
+            "    try: call()\n"
+            "    except capi.AxhelError as e: print(e.status)\n")
+    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True)
+    assert (r.returncode, r.stdout) == (0, "1\n1\n"), r.stderr
