@@ -95,15 +95,22 @@ def build_tools(force=False):
 
 
 def build_pyext(force=False):
-    """The Python extension ``axhel_b200/_fastcall.so`` (pyext/fastcall.c)."""
+    """The Python extension ``axhel_b200/_fastcall.so`` (pyext/fastcall.c).
+    Without a C compiler or Python's headers it is left out: the binding calls
+    through ctypes then, and C and C++ callers need none of it."""
     import sysconfig
 
     src = os.path.join(PKG, "pyext", "fastcall.c")
     out = os.path.join(PKG, "_fastcall.so")
     if not force and os.path.exists(out) and os.path.getmtime(out) >= os.path.getmtime(src):
         return
-    cmd = ["gcc", "-O2", "-Wall", "-Wextra", "-shared", "-fPIC", "-I" + sysconfig.get_paths()["include"], src, "-o",
-           out + ".tmp"]
+    include = sysconfig.get_paths()["include"]
+    if not shutil.which("gcc") or not os.path.exists(os.path.join(include, "Python.h")):
+        sys.stderr.write(f"{os.path.basename(out)} not built: no gcc, or no Python.h in {include}; calls go through ctypes\n")
+        if os.path.exists(out):
+            os.remove(out)  # of an older source
+        return
+    cmd = ["gcc", "-O2", "-Wall", "-Wextra", "-shared", "-fPIC", "-I" + include, src, "-o", out + ".tmp"]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"extension build failed: {' '.join(cmd)}\n{r.stdout}\n{r.stderr}")

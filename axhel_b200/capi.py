@@ -12,8 +12,13 @@ import os
 
 try:
     from ._fastcall import call as _fast, handle_type as _handle_type
-except ImportError as e:
-    raise RuntimeError("axhel_b200/_fastcall.so not built (run python -m axhel_b200.build)") from e
+except ImportError:
+    # not built, or for another Python: every call goes through ctypes
+    def _fast(*args):
+        return None
+
+    def _handle_type(cls):
+        pass
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "libaxhel.so")

@@ -106,3 +106,37 @@ def test_replaced_handle_is_the_one_passed():
             "    except capi.AxhelError as e: print(e.status)\n")
     r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True)
     assert (r.returncode, r.stdout) == (0, "1\n1\n"), r.stderr
+
+
+WITHOUT = "import sys\nsys.modules['axhel_b200._fastcall'] = None\n"
+
+
+def test_calls_without_the_extension():
+    code = WITHOUT + ("from axhel_b200 import capi\n"
+                      "capi.add(0, 0, 0, 0, 97)\n"
+                      "capi.tensor_product(0, 0, 0, 0, 0, 0, 0, 0, 0, [97])\n"
+                      "try: capi.forward_batch([], 8, 8, 1)\n"
+                      "except capi.AxhelError as e: print(e.status)\n"
+                      "try: capi.mul(0, 0, 0, None, 17, 1)\n"
+                      "except capi.C.ArgumentError: print('refused')\n")
+    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True)
+    assert (r.returncode, r.stdout) == (0, "1\nrefused\n"), r.stderr
+
+
+@pytest.mark.parametrize("missing", ["headers", "compiler"])
+def test_build_without_python_headers_or_compiler(tmp_path, monkeypatch, capsys, missing):
+    """The library builds for C and C++ callers; Python's go through ctypes."""
+    from axhel_b200 import build
+
+    (tmp_path / "pyext").mkdir()
+    (tmp_path / "pyext" / "fastcall.c").write_text("#include <Python.h>\n")
+    monkeypatch.setattr(build, "PKG", str(tmp_path))
+    if missing == "headers":
+        import sysconfig
+
+        monkeypatch.setattr(sysconfig, "get_paths", lambda: {"include": str(tmp_path)})
+    else:
+        monkeypatch.setenv("PATH", str(tmp_path))
+    build.build_pyext()
+    assert not (tmp_path / "_fastcall.so").exists()
+    assert "_fastcall" in capsys.readouterr().err
