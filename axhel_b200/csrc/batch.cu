@@ -571,7 +571,7 @@ axhel_status_t batch_build(const axhel_job_t* jobs, uint64_t n_jobs, unsigned ch
     std::vector<BatchJob> bj(n_jobs);
     std::vector<std::vector<const ModCtx*>> ctxs(n_jobs);
     std::vector<std::vector<uint64_t>> scal(n_jobs);
-    std::vector<uint32_t> n_fp(n_jobs, 0);  // moduli with FP64 forms
+    std::vector<uint32_t> n_fp(n_jobs, 0), n_form(n_jobs, 0);  // moduli with the FP64 form, with that or the relaxed one
     uint64_t done_total = 0;
     for (uint64_t i = 0; i < n_jobs; ++i) {
         const axhel_job_t& J = jobs[i];
@@ -581,6 +581,7 @@ axhel_status_t batch_build(const axhel_job_t* jobs, uint64_t n_jobs, unsigned ch
         if (st) return st;
         for (uint32_t m = 0; m < J.n_ntts; ++m) {
             n_fp[i] += !J.ntts[m]->external && J.ntts[m]->q < kFpModulusEnd;
+            n_form[i] += has_forms(J.ntts[m]);
             ctxs[i].push_back(J.ntts[m]->dctx);
             if (held) held->push_back(J.ntts[m]);
         }
@@ -672,11 +673,12 @@ axhel_status_t batch_build(const axhel_job_t* jobs, uint64_t n_jobs, unsigned ch
     }
     // the arithmetics of every entry, from its job's: a chain's inverse feeds
     // a MulMod / FMAMod, which takes any representative; lazy forwards run in
-    // FP64 where a quarter of the moduli or more have it
+    // FP64 where a quarter of the moduli or more have it; jobs without such
+    // moduli in the kernels of the reference's butterflies
     std::vector<uint32_t> ent_flags(ent.size(), 0), ent_forms(ent.size(), kFormsExact);
     for (size_t k = 0; k < ent.size(); ++k) {
         const BatchJob& b = bj[ent[k].job];
-        if (b.kind >= kJobAdd) continue;
+        if (b.kind >= kJobAdd || n_form[ent[k].job] == 0) continue;
         const bool chain = b.kind == kJobChainMul || b.kind == kJobChainFma, inverse = ent_cls[k] == kClsInv;
         const bool lazy_fp = 4 * n_fp[ent[k].job] >= b.nmods;
         uint32_t& f = ent_flags[k];

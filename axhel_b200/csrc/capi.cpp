@@ -106,7 +106,7 @@ ModCtx make_header(const axhel_ntt_ctx* c, unsigned char* base, uint64_t inv_las
     // Caller-provided tables keep the reference's arithmetic: nothing is
     // known of their entries.
     if (c->external) return h;
-    h.arith = c->q < kFpModulusEnd ? 2 : (c->q < kRelaxedModulusEnd ? 1 : 0);
+    h.arith = c->q < kFpModulusEnd ? 2 : (has_forms(c) ? 1 : 0);
     if (h.arith == 2) {
         const auto centred = [&](uint64_t w) { return w > c->q / 2 ? -(double)(c->q - w) : (double)w; };
         h.fq = (double)c->q;
@@ -457,6 +457,19 @@ uint64_t fp_moduli(const axhel_ntt_t* ntts, uint64_t n_ntts)
 }
 bool fp_any(const axhel_ntt_t* ntts, uint64_t n_ntts) { return fp_moduli(ntts, n_ntts) != 0; }
 
+// Whether any modulus has another form than the reference's butterflies: the
+// others keep the plan that was tuned for those (16 registers per thread in the
+// 7-stage passes, which the relaxed modes do not have).  60-bit moduli, us, the
+// narrowed plan of the relaxed modes then the tuned one: 225 limbs of N = 2^15
+// forward 95 and 91, inverse 98.5 and 99.3, chain 206 and 199, product 210 and
+// 192; 768 limbs of 2^16 562 and 565, 587 and 598, 1300 and 1299, 1274 and 1245.
+bool any_form(const axhel_ntt_t* ntts, uint64_t n_ntts)
+{
+    for (uint64_t i = 0; i < n_ntts; ++i)
+        if (has_forms(ntts[i])) return true;
+    return false;
+}
+
 // Whether a quarter of the moduli or more have FP64 forms.
 bool fp_share(const axhel_ntt_t* ntts, uint64_t n_ntts) { return 4 * fp_moduli(ntts, n_ntts) >= n_ntts; }
 
@@ -554,7 +567,7 @@ axhel_status_t transform(bool inverse, const axhel_ntt_t* ntts, uint64_t n_ntts,
     // normalized output: every pass may work on other representatives; a lazy
     // forward takes the same kernels' lazy FP64 form for the moduli it covers
     const bool lazy_fp = !norm && !inverse && (count << a.logn) >= kLazyFpWords && fp_share(ntts, n_ntts);
-    const bool relaxed = (norm || lazy_fp) && plan_relax(plan);
+    const bool relaxed = (norm || lazy_fp) && any_form(ntts, n_ntts) && plan_relax(plan);
     const uint32_t relax = relaxed ? (norm ? (uint32_t)kRelaxOut : (uint32_t)kLazyFp) : 0u;
     return run_plan(inverse, plan, a, operand, result, first, last, relax, S(stream));
 }
@@ -592,7 +605,8 @@ axhel_status_t chain(const axhel_ntt_t* ntts, uint64_t n_ntts, uint64_t* result,
     NttPlan inv = plan_for(true, logn, count);
     // the op takes any representative of the inverse's output, and a
     // normalized forward may work on any
-    const bool relaxable = ((count << logn) >= kRelaxIntWords || fp_any(ntts, n_ntts)) && plan_relax(inv);
+    const bool relaxable =
+        ((count << logn) >= kRelaxIntWords ? any_form(ntts, n_ntts) : fp_any(ntts, n_ntts)) && plan_relax(inv);
     const uint32_t relax_in = relaxable ? (uint32_t)kRelaxIn : 0u;
     const uint32_t relax_out = relaxable && out_f != 4 ? (uint32_t)kRelaxOut : 0u;
     // forward passes after the fused one: the inverse's earlier passes, reversed
@@ -686,7 +700,8 @@ axhel_status_t product(const axhel_ntt_t* ntts, uint64_t n_ntts, uint64_t* resul
     cudaStream_t s = S(stream);
     // the MulMod takes any representative of the forward's output, and a
     // normalized inverse may work on any
-    const bool relaxable = ((count << logn) >= kRelaxIntWords || fp_any(ntts, n_ntts)) && plan_relax(inv);
+    const bool relaxable =
+        ((count << logn) >= kRelaxIntWords ? any_form(ntts, n_ntts) : fp_any(ntts, n_ntts)) && plan_relax(inv);
     const uint32_t relax_in = relaxable ? (uint32_t)kRelaxIn : 0u;
     const uint32_t relax_out = relaxable && out_f != 2 ? (uint32_t)kRelaxOut : 0u;
     // fused: forward last pass -> MulMod -> inverse first pass (register depth 3:

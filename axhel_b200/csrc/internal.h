@@ -155,3 +155,11 @@ struct axhel_ntt_ctx {
     bool external = false;                     // tables supplied by the caller (axhel_cuda_ntt_create_external)
     const axhel_impl::ModCtx* dctx = nullptr;  // device address of the ModCtx header
 };
+
+namespace axhel_impl {
+
+// Whether the context's modulus has the FP64 or the relaxed integer form
+// (ModCtx::arith != 0).
+inline bool has_forms(const axhel_ntt_ctx* c) { return !c->external && c->q < kRelaxedModulusEnd; }
+
+}  // namespace axhel_impl
