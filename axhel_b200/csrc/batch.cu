@@ -522,7 +522,7 @@ static void set_specialized(ClassLaunch& L, const BatchJob& b, const std::vector
     // the job's passes agree on the arithmetic (batch_build): run them at the
     // register depth that holds it, or as class launches
     const bool forms = (L.first.flags & (kRelaxOut | kRelaxIn | kLazyFp)) != 0;
-    if (forms && !plan_relax(inv)) return;
+    if (forms && !plan_relax(true, b.logn, inv)) return;
     if (pc.chain) {
         if (inv.npass < 2) return;
         PassCfg fc = inv.pass[inv.npass - 1];
@@ -544,7 +544,7 @@ static void set_specialized(ClassLaunch& L, const BatchJob& b, const std::vector
         return;
     }
     NttPlan pl = pc.inv ? inv : plan_for(false, b.logn, b.count);
-    if (forms && !plan_relax(pl)) return;
+    if (forms && !plan_relax(pc.inv, b.logn, pl)) return;
     uint32_t s0 = 0;
     for (int i = 0; i < pl.npass; ++i) {
         if (s0 == pc.s0 && pl.pass[i].lg == (int)pc.lg) {

@@ -567,7 +567,7 @@ axhel_status_t transform(bool inverse, const axhel_ntt_t* ntts, uint64_t n_ntts,
     // normalized output: every pass may work on other representatives; a lazy
     // forward takes the same kernels' lazy FP64 form for the moduli it covers
     const bool lazy_fp = !norm && !inverse && (count << a.logn) >= kLazyFpWords && fp_share(ntts, n_ntts);
-    const bool relaxed = (norm || lazy_fp) && any_form(ntts, n_ntts) && plan_relax(plan);
+    const bool relaxed = (norm || lazy_fp) && any_form(ntts, n_ntts) && plan_relax(inverse, a.logn, plan);
     const uint32_t relax = relaxed ? (norm ? (uint32_t)kRelaxOut : (uint32_t)kLazyFp) : 0u;
     return run_plan(inverse, plan, a, operand, result, first, last, relax, S(stream));
 }
@@ -606,7 +606,7 @@ axhel_status_t chain(const axhel_ntt_t* ntts, uint64_t n_ntts, uint64_t* result,
     // the op takes any representative of the inverse's output, and a
     // normalized forward may work on any
     const bool relaxable =
-        ((count << logn) >= kRelaxIntWords ? any_form(ntts, n_ntts) : fp_any(ntts, n_ntts)) && plan_relax(inv);
+        ((count << logn) >= kRelaxIntWords ? any_form(ntts, n_ntts) : fp_any(ntts, n_ntts)) && plan_relax(true, logn, inv);
     const uint32_t relax_in = relaxable ? (uint32_t)kRelaxIn : 0u;
     const uint32_t relax_out = relaxable && out_f != 4 ? (uint32_t)kRelaxOut : 0u;
     // forward passes after the fused one: the inverse's earlier passes, reversed
@@ -701,7 +701,7 @@ axhel_status_t product(const axhel_ntt_t* ntts, uint64_t n_ntts, uint64_t* resul
     // the MulMod takes any representative of the forward's output, and a
     // normalized inverse may work on any
     const bool relaxable =
-        ((count << logn) >= kRelaxIntWords ? any_form(ntts, n_ntts) : fp_any(ntts, n_ntts)) && plan_relax(inv);
+        ((count << logn) >= kRelaxIntWords ? any_form(ntts, n_ntts) : fp_any(ntts, n_ntts)) && plan_relax(true, logn, inv);
     const uint32_t relax_in = relaxable ? (uint32_t)kRelaxIn : 0u;
     const uint32_t relax_out = relaxable && out_f != 2 ? (uint32_t)kRelaxOut : 0u;
     // fused: forward last pass -> MulMod -> inverse first pass (register depth 3:

@@ -99,9 +99,10 @@ bool pass_supported(const PassCfg& cfg);
 // Whether the pass's kernels hold the relaxed modes: kRelaxOut / kRelaxIn are
 // set on the passes of a call only if all of them do.
 bool pass_relaxable(const PassCfg& cfg);
-// The plan with its passes at the register depth of the relaxed modes, where
-// that fits every pass; false (and `p` as it was) if not.
-bool plan_relax(NttPlan& p);
+// The plan of (inverse, logN) with its passes at the register depth of the
+// relaxed modes, where that fits every pass; false (and `p` as it was) if not.
+// A plan set by axhel_cuda_plan_set is left as it is.
+bool plan_relax(bool inverse, uint32_t logn, NttPlan& p);
 
 // Single-launch forms of a few limbs, one thread-block cluster per limb
 // (ntt_cluster.cu): first-pass (transforms) or row (fused chains) stages,

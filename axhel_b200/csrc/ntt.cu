@@ -96,9 +96,15 @@ bool pass_supported(const PassCfg& c)
 
 bool pass_relaxable(const PassCfg& c) { return relaxed_compiled(c.lg, c.lr); }
 
-bool plan_relax(NttPlan& p)
+bool plan_relax(bool inverse, uint32_t logn, NttPlan& p)
 {
     NttPlan r = p;
+    if (plan_overridden(inverse, logn)) {
+        // set by the caller: as it is, or with the reference's butterflies
+        for (int i = 0; i < p.npass; ++i)
+            if (!pass_relaxable(p.pass[i])) return false;
+        return true;
+    }
     for (int i = 0; i < p.npass; ++i) {
         PassCfg& c = r.pass[i];
         // A pass tuned with 16 registers per thread takes twice the threads

@@ -430,10 +430,16 @@ axhel_status_t axhel_cuda_tensor_product(uint64_t* r0, uint64_t* r1, uint64_t* r
 
 /* Force the pass split for (inverse, log2 N): npass passes of lg[i] stages
  * (sum == log2 N), lr[i] register stages and tg[i] groups per CTA.
- * npass == 0 restores the default.  Used by the autotuner. */
+ * npass == 0 restores the default.  Used by the autotuner.  Calls run it as
+ * set, but for the fused pass of a chain or product, which has at most 3
+ * register stages. */
 axhel_status_t axhel_cuda_plan_set(int inverse, uint32_t log_degree, uint32_t npass, const uint32_t* lg,
                                    const uint32_t* lr, const uint32_t* tg);
-/* Reads the plan used for (inverse, log2 N, count limbs); arrays of >= 3. */
+/* Reads the plan used for (inverse, log2 N, count limbs); arrays of >= 3.
+ * Where it was not set by axhel_cuda_plan_set, calls whose output or inner
+ * values are normalized and that have a modulus below 2^59 with library-made
+ * tables run its passes with 3 register stages, those of 4 with half the
+ * groups per CTA where that leaves 8 or more. */
 axhel_status_t axhel_cuda_plan_get(int inverse, uint32_t log_degree, uint64_t count, uint32_t* npass, uint32_t* lg,
                                    uint32_t* lr, uint32_t* tg);
 /* Single-launch forms of a few limbs (new; no counterpart in the reference,

@@ -53,3 +53,40 @@ def test_exact_moduli_run_the_tuned_plan(cuda, oracle, bits, external):
     assert (run["inv"], run["fwd"]) == ({plan[1]}, {plan[1]})
     want = oracle.inverse(oracle.mul(oracle.forward(x[0], q, fwd, 1, 4), x[0], q, 4), q, inv, ninv, 2, 1)
     np.testing.assert_array_equal(host(o, n), want)
+
+
+# 16 registers per thread (the reference's butterflies), and 8 with tiles wider
+# than the relaxed modes' own
+@pytest.mark.parametrize("bits", [45, 55])
+@pytest.mark.parametrize("col,row", [((7, 4, 16), (7, 4, 16)), ((7, 3, 32), (7, 3, 16))])
+def test_forced_plans_run_as_set(cuda, oracle, bits, col, row):
+    n, count = 16384, 40
+    q, (fwd, inv, ninv), t = make(cuda, oracle, n, bits, False)
+    rng = np.random.default_rng(bits)
+    x, m = (rng.integers(0, q, (count, n), dtype=np.uint64) for _ in range(2))
+    d, e, o = dev(x), dev(m), dev_empty(count * n)
+    want = {
+        "forward": lambda a, b: oracle.forward(a, q, fwd, 1, 1),
+        "inverse": lambda a, b: oracle.inverse(a, q, inv, ninv, 1, 1),
+        "chain": lambda a, b: oracle.forward(oracle.mul(oracle.inverse(a, q, inv, ninv, 1, 2), b, q, 2), q, fwd, 1, 1),
+        "product": lambda a, b: oracle.inverse(oracle.mul(oracle.forward(a, q, fwd, 1, 4), b, q, 4), q, inv, ninv, 2, 1),
+    }
+    call = {
+        "forward": lambda: cuda.forward_batch([t], ptr(o), ptr(d), count, 1, 1),
+        "inverse": lambda: cuda.inverse_batch([t], ptr(o), ptr(d), count, 1, 1),
+        "chain": lambda: cuda.chain_mul_batch([t], ptr(o), ptr(d), ptr(e), count, 1, 1),
+        "product": lambda: cuda.product_batch([t], ptr(o), ptr(d), ptr(e), count, 1, 1),
+    }
+    passes = {"forward": {"fwd": {col, row}, "inv": set()}, "inverse": {"fwd": set(), "inv": {row, col}},
+              "chain": {"fwd": {row}, "inv": {row}}, "product": {"fwd": {col}, "inv": {col}}}
+    try:
+        cuda.plan_set(False, 14, [col, row])
+        cuda.plan_set(True, 14, [row, col])
+        for name in want:
+            assert passes_run(cuda, call[name]) == passes[name], name
+            got = host(o).reshape(count, n)
+            for i in (0, count - 1):
+                np.testing.assert_array_equal(got[i], want[name](x[i], m[i]), err_msg=f"{name}: limb {i}")
+    finally:
+        cuda.plan_set(False, 14, [])
+        cuda.plan_set(True, 14, [])
