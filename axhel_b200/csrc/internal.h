@@ -118,6 +118,7 @@ bool cluster_cfg_valid(int kind, uint32_t logn, const ClusterCfg& c);
 // The cluster form for (kind, logN, limbs), if it applies.
 bool cluster_plan(int kind, uint32_t logn, uint64_t count, ClusterCfg* out);
 void cluster_plan_override(int kind, uint32_t logn, const ClusterCfg* c);  // nullptr clears
+bool cluster_plan_overridden(int kind, uint32_t logn);
 ClusterCfg cluster_plan_current(int kind, uint32_t logn);
 // The autotuner's table entry (`K` lines of ntt_plans.txt), between the
 // override and the built-in choice.

@@ -769,6 +769,11 @@ void cluster_plan_override(int kind, uint32_t logn, const ClusterCfg* c)
     g_set[kind][logn].store(c != nullptr, std::memory_order_release);
 }
 
+bool cluster_plan_overridden(int kind, uint32_t logn)
+{
+    return kind >= 0 && kind <= 3 && logn <= 17 && g_set[kind][logn].load(std::memory_order_acquire);
+}
+
 ClusterCfg cluster_plan_current(int kind, uint32_t logn)
 {
     if (kind < 0 || kind > 3 || logn > 17) return ClusterCfg{0, 0, 0, 0};

@@ -240,3 +240,36 @@ def test_fused_cluster_chains_bitexact(cuda, oracle, logn):
     finally:
         for kind in (cuda.CLUSTER_CHAIN, cuda.CLUSTER_PRODUCT):
             cuda.cluster_plan_set(kind, logn)
+
+
+@pytest.mark.parametrize("kind", ["chain", "product"])
+def test_cluster_shape_set_by_hand_is_used(cuda, oracle, kind):
+    """Moduli below 2^50, 66 limbs of N = 2^12: by default the FP64 passes; a
+    cluster shape set for that many limbs takes its place, with the same bits."""
+    logn, count = 12, 66
+    n = 1 << logn
+    q = oracle.find_ntt_prime_near(n, 45, 1, 1)
+    t = cuda.NTT(n, q, oracle.find_primitive_root(n, q))
+    rng = np.random.default_rng(66)
+    d, e = (dev(rng.integers(0, q, count * n, dtype=np.uint64)) for _ in range(2))
+    k = cuda.CLUSTER_CHAIN if kind == "chain" else cuda.CLUSTER_PRODUCT
+    f = cuda.chain_mul_batch if kind == "chain" else cuda.product_batch
+
+    def run():
+        o = dev_empty(count * n)
+        cuda.profile_enable(True)
+        cuda.profile_report()
+        f([t], ptr(o), ptr(d), ptr(e), count, 1, 1)
+        names = list(cuda.profile_report())
+        cuda.profile_enable(False)
+        return host(o), names
+
+    want, names = run()
+    assert not any("cluster" in s for s in names)
+    try:
+        cuda.cluster_plan_set(k, logn, 6, 2, 8, count)
+        got, names = run()
+    finally:
+        cuda.cluster_plan_set(k, logn)
+    assert names == [f"ntt_{kind}_cluster lgr=6 lr=2 c=8"]
+    np.testing.assert_array_equal(got, want)
