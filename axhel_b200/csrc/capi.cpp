@@ -589,10 +589,14 @@ axhel_status_t chain(const axhel_ntt_t* ntts, uint64_t n_ntts, uint64_t* result,
     if (op == kChainFma && !scalars) return fail(AXHEL_ERR_INVALID, "null scalars");
     c.pass.count = count;
     const uint32_t logn = c.pass.logn;
+    // The first of several passes overwrites a vector that lies in the result;
+    // the one-launch forms have read all of it by then, so such a call takes
+    // one where there is one.
+    const bool vec_in_result = vec && vec == result;
     // a few limbs: the whole chain in one launch, one cluster per limb
     ClusterCfg cc;
     if (!plan_overridden(true, logn) && cluster_plan(kClusterChain, logn, count, &cc) &&
-        !fp_passes_win(kClusterChain, ntts, n_ntts, logn, count)) {
+        (vec_in_result || !fp_passes_win(kClusterChain, ntts, n_ntts, logn, count))) {
         c.pass.src = operand;
         c.pass.dst = result;
         c.pass.flags = (in_f == 4 ? (uint32_t)kPreCsub2q : 0u) | (out_f != 4 ? (uint32_t)kPostNorm : 0u);
@@ -606,6 +610,8 @@ axhel_status_t chain(const axhel_ntt_t* ntts, uint64_t n_ntts, uint64_t* result,
         if (!cluster_unschedulable(e)) return cuda_fail(e, "chain (cluster)");
     }
     NttPlan inv = plan_for(true, logn, count);
+    if (vec_in_result && inv.npass > 1 && logn <= 12 && !plan_overridden(true, logn))
+        inv = NttPlan{1, {PassCfg{(int)logn, logn < 3 ? (int)logn : 3, 1}}};
     // the op takes any representative of the inverse's output, and a
     // normalized forward may work on any
     const bool relaxable =

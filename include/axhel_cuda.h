@@ -138,7 +138,9 @@ axhel_status_t axhel_cuda_ntt_inverse_batch(const axhel_ntt_t* ntts, uint64_t n_
  *   ComputeInverse(x, x, in_f, 2); EltwiseMulMod(x, x, m, N, q, 2);
  *   ComputeForward(x, x, 1, out_f)
  * per limb).  `multiplicand` has the same layout as `operand`, values in
- * [0, 2q).  in_f == 4 fuses EltwiseReduceMod(4,2) ahead of the inverse. */
+ * [0, 2q); it may be `result` for N <= 2^12 (as long as no pass plan was set
+ * for that degree), not for larger N, where the first pass writes `result`.
+ * in_f == 4 fuses EltwiseReduceMod(4,2) ahead of the inverse. */
 axhel_status_t axhel_cuda_ntt_chain_mul_batch(const axhel_ntt_t* ntts, uint64_t n_ntts, uint64_t* result,
                                               const uint64_t* operand, const uint64_t* multiplicand, uint64_t count,
                                               uint64_t input_mod_factor, uint64_t output_mod_factor, void* stream);
@@ -180,7 +182,8 @@ axhel_status_t axhel_cuda_ntt_product_batch(const axhel_ntt_t* ntts, uint64_t n_
  *   ComputeInverse(x, x, in_f, 2); EltwiseFMAMod(x, x, scalars[i % n_ntts], addend_or_null, N, q, 2);
  *   ComputeForward(x, x, 1, out_f)
  * scalars is a HOST array of n_ntts values in [0, 2q); addend (device, same
- * layout as operand, values in [0, 2q)) may be NULL. */
+ * layout as operand, values in [0, 2q)) may be NULL, or `result` where a
+ * multiplicand of axhel_cuda_ntt_chain_mul_batch may be. */
 axhel_status_t axhel_cuda_ntt_chain_fma_batch(const axhel_ntt_t* ntts, uint64_t n_ntts, uint64_t* result,
                                               const uint64_t* operand, const uint64_t* scalars, const uint64_t* addend,
                                               uint64_t count, uint64_t input_mod_factor, uint64_t output_mod_factor,

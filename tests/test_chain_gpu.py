@@ -148,3 +148,31 @@ def test_forward_mul_and_mul_inverse_match_call_sequences(cuda, oracle, n, count
         cuda.forward_mul_batch(ntts, ptr(dm), ptr(d), ptr(dm), count)
     with pytest.raises(cuda.AxhelError):
         cuda.mul_inverse_batch(ntts, ptr(dm), ptr(d), ptr(dm), count, 1)
+
+
+# One launch holds the whole limb up to N = 2^12, whatever the batch size, and
+# for few limbs of larger ones: the vector may be the result buffer there.
+@pytest.mark.parametrize("n,count", [(1024, 3), (4096, 2), (4096, 64), (4096, 70), (4096, 600), (8192, 32)])
+@pytest.mark.parametrize("bits", [45, 55, 60])
+def test_chain_vector_is_the_result(cuda, oracle, n, count, bits):
+    q = oracle.find_ntt_prime_near(n, bits, 1, 1)
+    psi = oracle.find_primitive_root(n, q)
+    t = cuda.NTT(n, q, psi)
+    fwd, inv, ninv = oracle.tables(n, q, psi)
+    rng = np.random.default_rng(n + count + bits)
+    x, m = (rng.integers(0, q, (count, n), dtype=np.uint64) for _ in range(2))
+    some = sorted({0, 1, count // 2, count - 2, count - 1})
+    y = {i: oracle.inverse(x[i], q, inv, ninv, 1, 2) for i in some}
+    for out_f in (1, 4):
+        d, r = dev(x), dev(m)
+        cuda.chain_mul_batch([t], ptr(r), ptr(d), ptr(r), count, 1, out_f)
+        got = host(r).reshape(count, n)
+        for i in some:
+            np.testing.assert_array_equal(got[i], oracle.forward(oracle.mul(y[i], m[i], q, 2), q, fwd, 1, out_f),
+                                          err_msg=f"mul, out_f={out_f}, limb {i}")
+        d, r = dev(x), dev(m)
+        cuda.chain_fma_batch([t], ptr(r), ptr(d), [q // 3], ptr(r), count, 1, out_f)
+        got = host(r).reshape(count, n)
+        for i in some:
+            np.testing.assert_array_equal(got[i], oracle.forward(oracle.fma(y[i], q // 3, m[i], q, 2), q, fwd, 1, out_f),
+                                          err_msg=f"fma, out_f={out_f}, limb {i}")
