@@ -3,6 +3,7 @@
 
 #include <mutex>
 
+#include "device_once.h"
 #include "launch.h"
 #include "ntt_table.cuh"
 
@@ -16,7 +17,7 @@ constexpr int kSmemPlain = 2;  // third "pair" column
 // Two limbs per thread halve the CTAs: only where they still fill the GPU.
 constexpr uint64_t kPairThreadsPerSm = 1024;
 
-bool g_smem_set[kFnKinds][2][3][2][kMaxLG + 1][kMaxLR + 1];
+DeviceOnce g_smem_set[kFnKinds][2][3][2][kMaxLG + 1][kMaxLR + 1];
 
 std::mutex g_attr_mu;
 
@@ -27,14 +28,14 @@ cudaError_t ensure_smem(Fn fn, FnKind kind, bool relax, int column, bool row, co
 {
     const size_t bytes = smem_bytes(c) << (column == 1);
     if (bytes <= 48 * 1024) return cudaSuccess;
-    std::lock_guard<std::mutex> lk(g_attr_mu);
+    int dev = 0;
+    const cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
     // Set to the maximum once per kernel; cheaper than tracking each size.
-    bool& done = g_smem_set[kind][relax][column][row][c.lg][c.lr];
-    if (done) return cudaSuccess;
-    cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(fn),
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-    if (e == cudaSuccess) done = true;
-    return e;
+    return g_smem_set[kind][relax][column][row][c.lg][c.lr](dev, g_attr_mu, [&] {
+        return cudaFuncSetAttribute(reinterpret_cast<const void*>(fn), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    227 * 1024);
+    });
 }
 
 // Whether a launch's limbs run two per thread, pairs of the batch's groups of

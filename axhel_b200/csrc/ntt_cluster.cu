@@ -35,6 +35,7 @@
 #include <atomic>
 #include <mutex>
 
+#include "device_once.h"
 #include "launch.h"
 #include "ntt_kernels.cuh"
 
@@ -693,27 +694,23 @@ ClusterCfg current_cfg(int kind, uint32_t logn)
     }
     return c;
 }
-// per kernel and device: shared-memory / cluster-size attributes set (bit
-// `device`), read without the lock once set
+// per kernel and device: shared-memory / cluster-size attributes set
 std::mutex g_attr_mu;
-std::atomic<uint64_t> g_attr_done[kNumEntries][2][2] = {};
-std::atomic<uint64_t> g_fused_attr_done[kNumFused][2] = {};
+DeviceOnce g_attr_done[kNumEntries][2][2];
+DeviceOnce g_fused_attr_done[kNumFused][2];
 
 int entry_index(const Entry* e) { return (int)(e - kEntries); }
 int fused_index(const FusedEntry* e) { return (int)(e - kFused); }
 
 bool fused_kind(int kind) { return kind == kClusterChain || kind == kClusterProduct; }
 
-// Sets the launch attributes of `fn` once per device (bit `dev` of `done`).
-cudaError_t ensure_attrs(const void* fn, std::atomic<uint64_t>& done, int dev)
+// Sets the launch attributes of `fn` once per device.
+cudaError_t ensure_attrs(const void* fn, DeviceOnce& done, int dev)
 {
-    if (done.load(std::memory_order_acquire) >> dev & 1) return cudaSuccess;
-    std::lock_guard<std::mutex> lk(g_attr_mu);
-    if (done.load(std::memory_order_relaxed) >> dev & 1) return cudaSuccess;
-    cudaError_t err = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-    if (err == cudaSuccess) err = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (err == cudaSuccess) done.fetch_or(1ull << dev, std::memory_order_release);
-    return err;
+    return done(dev, g_attr_mu, [&] {
+        const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        return e != cudaSuccess ? e : cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    });
 }
 
 cudaError_t launch_cluster(const void* fn, void* args, uint64_t blocks, uint32_t threads, size_t smem, int csize,

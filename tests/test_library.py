@@ -216,3 +216,33 @@ print("ok")
 """
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, cwd=ROOT, timeout=120)
     assert r.returncode == 0 and "ok" in r.stdout, r.stderr[-2000:]
+
+
+def test_function_attributes_are_set_once_per_device(tmp_path):
+    """DeviceOnce, which the launchers key their kernels' attributes by: each
+    device of a process sets its own, failures are tried again."""
+    probe = tmp_path / "once.cpp"
+    probe.write_text("""
+#include <initializer_list>
+#include "device_once.h"
+enum Err { kOk = 0, kBad = 1 };
+int main()
+{
+    static axhel_impl::DeviceOnce once[2];
+    std::mutex mu;
+    int calls = 0;
+    auto set = [&] { ++calls; return kOk; };
+    for (int round = 0; round < 2; ++round)
+        for (int dev : {0, 1, 63})
+            if (once[0](dev, mu, set) != kOk || calls != (round ? 3 : (dev == 63 ? 3 : dev + 1))) return 1;
+    if (once[1](0, mu, [] { return kBad; }) != kBad) return 2;
+    if (once[1](0, mu, set) != kOk || calls != 4) return 3;
+    once[1](64, mu, set);
+    once[1](64, mu, set);
+    return calls == 6 ? 0 : 4;
+}
+""")
+    exe = tmp_path / "once"
+    subprocess.run(["g++", "-std=c++17", "-Wall", "-Wextra", "-Werror",
+                    "-I" + os.path.join(ROOT, "axhel_b200", "csrc"), str(probe), "-o", str(exe)], check=True)
+    assert subprocess.run([str(exe)]).returncode == 0
