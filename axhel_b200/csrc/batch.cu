@@ -874,10 +874,15 @@ ClassKernel pick_class_kernel(uint32_t cls, uint32_t lg)
 #define AXHEL_CLASS_ROW(CLS)                                                                                 \
     {class_kernel<CLS, 5, FORMS>(), class_kernel<CLS, 6, FORMS>(), class_kernel<CLS, 7, FORMS>(),            \
      class_kernel<CLS, 8, FORMS>(), class_kernel<CLS, 9, FORMS>()}
-    static const ClassKernel table[3][5] = {AXHEL_CLASS_ROW(kClsFwd), AXHEL_CLASS_ROW(kClsInv),
-                                            AXHEL_CLASS_ROW(kClsChain)};
+    static const ClassKernel fwd[5] = AXHEL_CLASS_ROW(kClsFwd), chain[5] = AXHEL_CLASS_ROW(kClsChain);
+    if (cls == kClsFwd) return fwd[lg - kBatchMinLG];
+    if (cls == kClsChain) return chain[lg - kBatchMinLG];
+    if constexpr (FORMS != kFormsLazy) {  // a form of forwards and of the chains' fused passes
+        static const ClassKernel inv[5] = AXHEL_CLASS_ROW(kClsInv);
+        if (cls == kClsInv) return inv[lg - kBatchMinLG];
+    }
 #undef AXHEL_CLASS_ROW
-    return cls < 3 ? table[cls][lg - kBatchMinLG] : ClassKernel{};
+    return ClassKernel{};
 }
 
 ClassKernel pick_class_kernel(uint32_t cls, uint32_t lg, uint32_t forms)

@@ -6,7 +6,8 @@ namespace axhel_impl {
 namespace {
 template <int LG, int LR, bool RELAX, int P, int SHAPE>
 struct Get {
-    static constexpr bool compiled = true, has_plain = true, shaped = false;
+    static constexpr bool compiled = true, has_plain = true, exact_pairs = true;
+    static constexpr Columns columns = kSameColumns;
     static ChainFn fn() { return ntt_chain_kernel<LG, LR, P != 0, RELAX, P == 2 ? 2 : 1>; }
 };
 }  // namespace

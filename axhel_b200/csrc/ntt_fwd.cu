@@ -1,4 +1,5 @@
-// The forward pass kernels (ntt_kernels.cuh).
+// The forward pass kernels (ntt_kernels.cuh); lazy forwards run one limb per
+// thread (pairs() in ntt.cu).
 #include "ntt_table.cuh"
 
 namespace axhel_impl {
@@ -6,7 +7,8 @@ namespace axhel_impl {
 namespace {
 template <int LG, int LR, bool RELAX, int P, int SHAPE>
 struct Get {
-    static constexpr bool compiled = true, has_plain = false, shaped = true;
+    static constexpr bool compiled = true, has_plain = false, exact_pairs = false;
+    static constexpr Columns columns = kOwnColumns;
     static PassFn fn()
     {
         if constexpr (P == 2) return ntt_pass_pair_kernel<false, LG, LR, RELAX, SHAPE>;

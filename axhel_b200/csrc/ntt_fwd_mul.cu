@@ -1,4 +1,5 @@
-// The forward pass kernels with the dyadic product (ntt_kernels.cuh).
+// The forward pass kernels with the dyadic product (ntt_kernels.cuh): the last pass of a
+// transform, on contiguous rows.
 #include "ntt_table.cuh"
 
 namespace axhel_impl {
@@ -6,7 +7,8 @@ namespace axhel_impl {
 namespace {
 template <int LG, int LR, bool RELAX, int P, int SHAPE>
 struct Get {
-    static constexpr bool compiled = true, has_plain = false, shaped = true;
+    static constexpr bool compiled = true, has_plain = false, exact_pairs = true;
+    static constexpr Columns columns = kNoColumns;
     static PassFn fn()
     {
         if constexpr (P == 2) return ntt_pass_mul_pair_kernel<false, LG, LR, RELAX, SHAPE>;

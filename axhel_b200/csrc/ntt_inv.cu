@@ -6,7 +6,8 @@ namespace axhel_impl {
 namespace {
 template <int LG, int LR, bool RELAX, int P, int SHAPE>
 struct Get {
-    static constexpr bool compiled = true, has_plain = false, shaped = true;
+    static constexpr bool compiled = true, has_plain = false, exact_pairs = true;
+    static constexpr Columns columns = kOwnColumns;
     static PassFn fn()
     {
         if constexpr (P == 2) return ntt_pass_pair_kernel<true, LG, LR, RELAX, SHAPE>;

@@ -730,7 +730,7 @@ __device__ __forceinline__ void run_rounds(uint64_t (&v)[1 << LR], uint64_t* smg
 
 // Group sizes and register depth compiled with the relaxed modes: 8 registers
 // per thread (16 would take 110-128 machine registers for the modes together).
-constexpr bool relaxed_compiled(int lg, int lr) { return lr == 3 && lg >= 4 && lg <= 13; }
+constexpr bool relaxed_compiled(int lg, int lr) { return lr == 3 && lg >= 4 && (1 << (lg - lr)) <= max_threads(lr); }
 
 // ------------------------------------------------------------------ kernels
 
@@ -868,7 +868,6 @@ __device__ __forceinline__ void pass_tile_as(const uint64_t* src, uint64_t* dst,
         bool stored = false;
         if constexpr (MUL && !INV) {
             if (flags & kPostMul) {
-                if constexpr (MODE == kFpLazy) fwd_output<MODE, LR>(v[p], false, cx);
                 mul_operand<MODE, LG, LR, LO_LAST, CG>(v[p], operand + (limb << logn) + p * pstep, t, gi, k, cx,
                                                        vec_ok, 32);
                 if constexpr (MODE == kFp) inv_output<MODE, LR>(v[p], true, cx);
@@ -939,7 +938,7 @@ __device__ __forceinline__ void pass_tile(const uint64_t* src, uint64_t* dst, co
                 });
                 return;
             }
-        } else if constexpr (!INV) {
+        } else if constexpr (!INV && !MUL) {  // (a product's output is normalized)
             if (kind == kFp && (flags & kLazyFp)) {
                 pass_tile_as<kFpLazy, INV, LG, LR, CG, MUL, P, SHAPE>(src, dst, cx, logn, s0, lgtg, limb, lstep,
                                                                tile_in_limb, flags, sm, operand);

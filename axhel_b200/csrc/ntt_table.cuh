@@ -34,6 +34,12 @@ const FnTable<PassFn>& inv_mul_table();
 const FnTable<ChainFn>& chain_table();
 const FnTable<ChainFn>& product_table();
 
+// What the launchers reach of a kind's kernels (its Get::): `compiled` register
+// depths, `has_plain` kernels, `exact_pairs` -- two limbs per thread without
+// kRelaxOut -- and kernels for strided columns: of their own, the same as for
+// contiguous rows, or none (no such pass).
+enum Columns : int { kNoColumns, kSameColumns, kOwnColumns };
+
 template <template <int, int, bool, int, int> class Get, class Fn, int LG, int LR, int SHAPE>
 void add_shape(FnTable<Fn>& t)
 {
@@ -41,26 +47,28 @@ void add_shape(FnTable<Fn>& t)
     t.at[0][0][row][LG][LR] = Get<LG, LR, false, 1, SHAPE>::fn();
     if constexpr (relaxed_compiled(LG, LR)) {
         t.at[1][0][row][LG][LR] = Get<LG, LR, true, 1, SHAPE>::fn();
-        t.at[0][1][row][LG][LR] = Get<LG, LR, false, 2, SHAPE>::fn();
+        if constexpr (Get<LG, LR, false, 1, SHAPE>::exact_pairs)
+            t.at[0][1][row][LG][LR] = Get<LG, LR, false, 2, SHAPE>::fn();
         t.at[1][1][row][LG][LR] = Get<LG, LR, true, 2, SHAPE>::fn();
     }
 }
 
 // Fills a table with Get<LG, LR, RELAX, P, SHAPE>::fn(); P limbs per thread, 0: plain.  Register-stage counts
-// compiled for each group size: LR = LG for tiny groups, otherwise 3, 4 and 5.
+// compiled for each group size: LR = LG for tiny groups, otherwise 3, 4 and 5
+// where a group's threads fit a CTA.
 template <template <int, int, bool, int, int> class Get, class Fn, int LG, int LR>
 void add_one(FnTable<Fn>& t)
 {
-    if constexpr (LR <= LG && Get<LG, LR, false, 1, kRowTiles>::compiled) {
+    using G = Get<LG, LR, false, 1, kRowTiles>;
+    if constexpr (LR <= LG && (1 << (LG - LR)) <= max_threads(LR) && G::compiled) {
         add_shape<Get, Fn, LG, LR, kRowTiles>(t);
-        if constexpr (Get<LG, LR, false, 1, kRowTiles>::shaped) {
-            add_shape<Get, Fn, LG, LR, kColumnTiles>(t);
-        } else {
+        if constexpr (G::columns == kOwnColumns) add_shape<Get, Fn, LG, LR, kColumnTiles>(t);
+        if constexpr (G::columns == kSameColumns) {
             for (auto& relax : t.at)
                 for (auto& pair : relax) pair[0][LG][LR] = pair[1][LG][LR];
         }
         t.plain[LG][LR] = t.at[0][0][1][LG][LR];
-        if constexpr (relaxed_compiled(LG, LR) && Get<LG, LR, false, 1, kRowTiles>::has_plain)
+        if constexpr (relaxed_compiled(LG, LR) && G::has_plain)
             t.plain[LG][LR] = Get<LG, LR, false, 0, kRowTiles>::fn();
     }
 }

@@ -53,6 +53,17 @@ def test_cpp_dropin_symbols_exported():
         assert sig in out, sig
 
 
+def test_no_kernel_is_compiled_that_no_call_launches():
+    """Forward pairs without relaxed modes, products in strided passes, lazy
+    inverses of the batch engine, groups of 2^13 with 1024 threads."""
+    out = subprocess.run(["nm", "-C", LIB], capture_output=True, text=True, check=True).stdout
+    names = set(re.findall(r"axhel_impl::((?:ntt|batch)_\w*kernel<[^>]*>)", out))
+    assert "ntt_pass_pair_kernel<false, 7, 3, true, 1>" in names and "batch_class_kernel<1, 7, 3, 1>" in names
+    dead = [n for n in names if re.match(r"ntt_pass_pair_kernel<false, \d+, 3, false|ntt_pass_mul\w*<.*, 1>|"
+                                         r"batch_class\w*<1, \d+, \d+, 2>|ntt_(pass|chain|product)\w*<.*\b13, 3, ", n)]
+    assert not dead, sorted(dead)
+
+
 def test_ctypes_load_and_cpu_side_calls():
     from axhel_b200 import capi
 
