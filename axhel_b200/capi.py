@@ -11,14 +11,9 @@ import ctypes as C
 import os
 
 try:
-    from ._fastcall import call as _fast, handle_type as _handle_type
+    from . import _fastcall
 except ImportError:
-    # not built, or for another Python: every call goes through ctypes
-    def _fast(*args):
-        return None
-
-    def _handle_type(cls):
-        pass
+    _fastcall = None  # not built, or for another Python: every call goes through ctypes
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "libaxhel.so")
@@ -106,8 +101,9 @@ def lib():
             raise RuntimeError(f"AXHEL CUDA library not built: {LIB_PATH} (run python -m axhel_b200.build)")
         L = C.CDLL(LIB_PATH)
         _declare(L)
-        for name in _HOT:
-            _hot[name] = C.cast(getattr(L, "axhel_cuda_" + name), vp).value
+        for name, kinds in _HOT.items():
+            _hot[name] = (_fastcall.entry(C.cast(getattr(L, "axhel_cuda_" + name), vp).value, kinds) if _fastcall
+                          else lambda *args: None)
         _lib = L
     return _lib
 
@@ -142,7 +138,7 @@ _ARRAYS = {"h": lambda ntts: (vp * len(ntts))(*[t.h.value for t in ntts]),
 
 
 class _Hot(dict):
-    """Addresses of the hot entry points; the first lookup loads the library."""
+    """The hot entry points' callables; the first lookup loads the library."""
 
     def __missing__(self, name):
         lib()
@@ -153,7 +149,7 @@ _hot = _Hot()
 
 
 def _call(name, where, *args):
-    st = _fast(_hot[name], _HOT[name], *args)
+    st = _hot[name](*args)
     if st is None:
         # an argument in another form than the extension's: ctypes converts or refuses it
         args = [_ARRAYS[k](x) if k in _ARRAYS else x for k, x in zip(_HOT[name], args)]
@@ -503,7 +499,8 @@ class NTT:
         _call("ntt_inverse", "ntt_inverse", self.hv, dst, src, in_f, out_f, stream)
 
 
-_handle_type(NTT)
+if _fastcall:
+    _fastcall.handle_type(NTT)
 
 
 def _seq(ntts):

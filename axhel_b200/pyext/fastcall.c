@@ -2,8 +2,8 @@
 //
 // A C-ABI call through ctypes costs 0.8-1.2 us for its argument conversions,
 // and an array of NTT handles 0.2 us per handle, against 2-3 us for the
-// launches behind it: a third of a small transform's host time.  call() passes
-// up to 14 integers (System V: every argument of these functions is an
+// launches behind it: a third of a small transform's host time.  A callable
+// made by entry() passes up to 14 integers (System V: every argument of these functions is an
 // integer or pointer of at most 64 bits in a register or 8-byte stack slot).
 //
 // It converts the plain argument forms only, each as ctypes converts it, and
@@ -12,6 +12,7 @@
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 #include <stdint.h>
+#include <string.h>
 
 #define MAX_ARGS 14
 #define MAX_ITEMS 256
@@ -67,25 +68,33 @@ static int from_ntt(PyObject* o, uint64_t* out)
     return r;
 }
 
-// call(address, kinds, *args) -> status, or None if an argument has another
-// form.  kinds: one letter per argument, "i" an integer, "p" an address, "h" a
-// list or tuple of NTT objects and "a" one of ints, these two passed as the
-// address of an array of their values (the caller passes their count too).
+// What an entry point's callable carries: its address and one letter per
+// argument, "i" an integer, "p" an address, "h" a list or tuple of NTT objects
+// and "a" one of ints, these two passed as the address of an array of their
+// values (the caller passes their count too).
+typedef struct {
+    fn_t fn;
+    int len;
+    char kinds[MAX_ARGS];
+} entry_t;
+
+// (*args) -> status, or None if an argument has another form.
 static PyObject* call(PyObject* self, PyObject* const* args, Py_ssize_t nargs)
 {
-    (void)self;
-    uint64_t a[MAX_ARGS] = {0}, items[MAX_ITEMS], addr;
+    const entry_t* entry = PyCapsule_GetPointer(self, NULL);
+    uint64_t a[MAX_ARGS] = {0}, items[MAX_ITEMS];
     uint64_t* heap[MAX_ARGS] = {0};
-    Py_ssize_t used = 0, len = 0;
-    const char* kinds = nargs >= 2 && PyUnicode_Check(args[1]) ? PyUnicode_AsUTF8AndSize(args[1], &len) : NULL;
-    if (!kinds || len > MAX_ARGS || nargs != len + 2 || from_int(args[0], &addr) != 1) {
-        if (!PyErr_Occurred()) PyErr_SetString(PyExc_TypeError, "call(address, kinds, one argument per kind)");
+    Py_ssize_t used = 0;
+    if (!entry) return NULL;
+    const Py_ssize_t len = entry->len;
+    if (nargs != len) {
+        PyErr_Format(PyExc_TypeError, "expected %zd arguments, got %zd", len, nargs);
         return NULL;
     }
     int r = 1;
     for (Py_ssize_t i = 0; r == 1 && i < len; ++i) {
-        PyObject* o = args[i + 2];
-        const char kind = kinds[i];
+        PyObject* o = args[i];
+        const char kind = entry->kinds[i];
         if (kind == 'i') {
             r = from_index(o, &a[i]);
             continue;
@@ -127,8 +136,7 @@ static PyObject* call(PyObject* self, PyObject* const* args, Py_ssize_t nargs)
     if (r == 1) {
         int32_t st;
         Py_BEGIN_ALLOW_THREADS
-        st = ((fn_t)(uintptr_t)addr)(a[0], a[1], a[2], a[3], a[4], a[5], a[6], a[7], a[8], a[9], a[10], a[11], a[12],
-                                     a[13]);
+        st = entry->fn(a[0], a[1], a[2], a[3], a[4], a[5], a[6], a[7], a[8], a[9], a[10], a[11], a[12], a[13]);
         Py_END_ALLOW_THREADS
         ret = PyLong_FromLong(st);
     } else if (r == 0) {
@@ -136,6 +144,38 @@ static PyObject* call(PyObject* self, PyObject* const* args, Py_ssize_t nargs)
     }
     for (int i = 0; i < MAX_ARGS; ++i) PyMem_Free(heap[i]);
     return ret;
+}
+
+static PyMethodDef call_def = {"call", (PyCFunction)(void (*)(void))call, METH_FASTCALL,
+                               "(*args) -> status, or None if an argument has another form"};
+
+static void free_entry(PyObject* capsule) { PyMem_Free(PyCapsule_GetPointer(capsule, NULL)); }
+
+// entry(address, kinds): the callable of an entry point.
+static PyObject* entry(PyObject* self, PyObject* args)
+{
+    (void)self;
+    unsigned long long address;
+    const char* kinds;
+    Py_ssize_t len;
+    if (!PyArg_ParseTuple(args, "Ks#", &address, &kinds, &len)) return NULL;
+    if (len > MAX_ARGS) {
+        PyErr_SetString(PyExc_ValueError, "too many arguments");
+        return NULL;
+    }
+    entry_t* e = PyMem_Malloc(sizeof *e);
+    if (!e) return PyErr_NoMemory();
+    e->fn = (fn_t)(uintptr_t)address;
+    e->len = (int)len;
+    memcpy(e->kinds, kinds, (size_t)len);
+    PyObject* capsule = PyCapsule_New(e, NULL, free_entry);
+    if (!capsule) {
+        PyMem_Free(e);
+        return NULL;
+    }
+    PyObject* f = PyCFunction_NewEx(&call_def, capsule, NULL);
+    Py_DECREF(capsule);
+    return f;
 }
 
 // handle_type(cls): the class whose objects an "h" list holds.
@@ -151,7 +191,7 @@ static PyObject* handle_type(PyObject* self, PyObject* cls)
 }
 
 static PyMethodDef methods[] = {
-    {"call", (PyCFunction)(void (*)(void))call, METH_FASTCALL, "call(address, kinds, *args) -> status or None"},
+    {"entry", entry, METH_VARARGS, "entry(address, kinds) -> callable"},
     {"handle_type", handle_type, METH_O, "handle_type(cls)"},
     {NULL, NULL, 0, NULL}};
 static struct PyModuleDef module = {PyModuleDef_HEAD_INIT, "_fastcall", NULL, -1, methods, NULL, NULL, NULL, NULL};
