@@ -46,13 +46,48 @@ def test_exact_moduli_run_the_tuned_plan(cuda, oracle, bits, external):
     plan = cuda.plan_get(True, 16, count)
     assert run["inv"] == set(plan)
     np.testing.assert_array_equal(host(o, n), oracle.inverse(x[0], q, inv, ninv, 1, 1))
-    # the passes beside the fused one, and a batch's
+    # the passes beside the fused one
     run = passes_run(cuda, lambda: cuda.chain_mul_batch([t], ptr(o), ptr(d), ptr(d), count, 1, 1))
     assert (run["inv"], run["fwd"]) == ({plan[0]}, {plan[0]})
     run = passes_run(cuda, lambda: cuda.product_batch([t], ptr(o), ptr(d), ptr(d), count, 1, 1))
     assert (run["inv"], run["fwd"]) == ({plan[1]}, {plan[1]})
     want = oracle.inverse(oracle.mul(oracle.forward(x[0], q, fwd, 1, 4), x[0], q, 4), q, inv, ninv, 2, 1)
     np.testing.assert_array_equal(host(o, n), want)
+
+
+@pytest.mark.parametrize("phased", [False, True])
+def test_batches_of_exact_moduli(cuda, oracle, phased):
+    """Jobs whose moduli have the reference's form only beside one that has others:
+    each as its direct call, launched by class (small jobs together, a large one
+    alone) and as one launch."""
+    jobs = [(n, bits, external, count, kind, out_f) for bits, external in [(60, False), (45, True), (45, False)]
+            for n, count in [(4096, 3), (32768, 40)]
+            for kind, out_f in [(cuda.JOB_FORWARD, 1), (cuda.JOB_INVERSE, 1), (cuda.JOB_CHAIN_MUL, 1),
+                                (cuda.JOB_CHAIN_MUL, 4)]]
+    rng = np.random.default_rng(60)
+    specs, outs, wants, ctx = [], [], [], {}
+    for n, bits, external, count, kind, out_f in jobs:
+        if (n, bits, external) not in ctx:
+            ctx[n, bits, external] = make(cuda, oracle, n, bits, external)
+        q, _, t = ctx[n, bits, external]
+        x, m = (dev(rng.integers(0, q, count * n, dtype=np.uint64)) for _ in range(2))
+        o, w = dev_empty(count * n), dev_empty(count * n)
+        specs.append(dict(kind=kind, ntts=[t], count=count, result=ptr(o), operand=ptr(x), vector=ptr(m), in_f=1,
+                          out_f=out_f, keep=(x, m)))
+        if kind == cuda.JOB_FORWARD:
+            cuda.forward_batch([t], ptr(w), ptr(x), count, 1, out_f)
+        elif kind == cuda.JOB_INVERSE:
+            cuda.inverse_batch([t], ptr(w), ptr(x), count, 1, out_f)
+        else:
+            cuda.chain_mul_batch([t], ptr(w), ptr(x), ptr(m), count, 1, out_f)
+        outs.append(o)
+        wants.append(w)
+    b = cuda.Batch(specs)
+    b.launch(phased=phased)
+    assert b.status() == 0
+    for o, w, j in zip(outs, wants, jobs):
+        np.testing.assert_array_equal(host(o), host(w), err_msg=str(j))
+    b.close()
 
 
 # 16 registers per thread (the reference's butterflies), and 8 with tiles wider
@@ -90,3 +125,96 @@ def test_forced_plans_run_as_set(cuda, oracle, bits, col, row):
     finally:
         cuda.plan_set(False, 14, [])
         cuda.plan_set(True, 14, [])
+
+
+def plans(logn):
+    """Splits of a forward, outermost stages first, whose passes hold the relaxed
+    modes (8 registers per thread, groups of 2^4 .. 2^12), with the narrowest,
+    a middle and the widest tiles; three passes; and passes without those modes."""
+    def widths(lg, most):
+        top = min(most, 512 >> (lg - 3))
+        return sorted({1, min(8, top), top})
+
+    out = [[(logn, 3, 1)]] if 4 <= logn <= 12 else []
+    for col in range(4, min(12, logn - 4) + 1):
+        row = logn - col
+        if not 4 <= row <= 12:
+            continue
+        cw, rw = widths(col, 1 << row), widths(row, 1 << col)
+        out += [[(col, 3, cw[i % len(cw)]), (row, 3, rw[-1 - i % len(rw)])] for i in range(3)]
+    if logn >= 12:
+        a, b = logn // 3, (logn - logn // 3) // 2
+        out += [[(a, 3, 8), (b, 3, 16), (logn - a - b, 3, 4)], [(b, 3, 16), (logn - a - b, 3, 1), (a, 3, 16)],
+                [(logn // 2, 4, 8), (logn - logn // 2, 3, 8)], [(logn // 2, 3, 8), (logn - logn // 2, 5, 4)]]
+    return out
+
+
+# An odd number of limbs per modulus (pairs and a last one alone), from N = 2^9 on
+# enough residues for two limbs per thread; moduli of every arithmetic, one with caller-provided tables.
+@pytest.mark.parametrize("logn,polys", [(6, 5), (9, 949), (11, 239), (12, 119), (13, 61), (14, 31), (16, 9),
+                                        (17, 7)])
+def test_forms_under_every_plan(cuda, oracle, logn, polys):
+    import torch
+
+    n, bits = 1 << logn, [(45, 1, 2), (50, 1, 1), (58, 1, 2), (60, 1, 2), (44, 1, 2)]
+    qs = [oracle.find_ntt_prime_near(n, *b) for b in bits]
+    psis = [oracle.find_primitive_root(n, q) for q in qs]
+    tabs = [oracle.tables(n, q, psi) for q, psi in zip(qs, psis)]
+    ntts = cuda.NTT.create_many(list(zip([n] * 4, qs, psis))) + [cuda.NTT(n, qs[4], tables=tabs[4])]
+    L, count = len(qs), len(qs) * polys
+    rng = np.random.default_rng(logn)
+    x4, m4, x2, m2 = (np.stack([rng.integers(0, f * qs[i % L], n, dtype=np.uint64) for i in range(count)])
+                      for f in (4, 4, 2, 2))
+    sc = [(2 * q) // 3 for q in qs]
+
+    def limbs(f):
+        return dev(np.concatenate([f(i, qs[i % L], *tabs[i % L]) for i in range(count)]))
+
+    fwd = lambda v, q, t, f=1: oracle.forward(v, q, t, 1, f)
+    inv = lambda v, q, t, ninv, f=1: oracle.inverse(v, q, t, ninv, 2, f)
+    lazy = [fwd(x4[i], qs[i % L], tabs[i % L][0], 4) for i in range(count)]
+    prod = [oracle.mul(lazy[i], m4[i], qs[i % L], 4) for i in range(count)]
+    back = [inv(x2[i], qs[i % L], tabs[i % L][1], tabs[i % L][2], 2) for i in range(count)]
+    d4, e4, d2, e2, o = dev(x4), dev(m4), dev(x2), dev(m2), dev_empty(count * n)
+    P, c = ptr, count
+    ops = {
+        "forward 4": (limbs(lambda i, *_: lazy[i]), lambda: cuda.forward_batch(ntts, P(o), P(d4), c, 4, 4)),
+        "forward 1": (limbs(lambda i, q, *_: oracle.reduce(lazy[i], q, 4, 1)),
+                      lambda: cuda.forward_batch(ntts, P(o), P(d4), c, 4, 1)),
+        "forward mul": (limbs(lambda i, *_: prod[i]), lambda: cuda.forward_mul_batch(ntts, P(o), P(d4), P(e4), c)),
+        "inverse 2": (limbs(lambda i, *_: back[i]), lambda: cuda.inverse_batch(ntts, P(o), P(d2), c, 2, 2)),
+        "inverse 1": (limbs(lambda i, q, *_: oracle.reduce(back[i], q, 2, 1)),
+                      lambda: cuda.inverse_batch(ntts, P(o), P(d2), c, 2, 1)),
+        "mul inverse": (limbs(lambda i, q, f, t, ninv: inv(oracle.mul(x4[i], m4[i], q, 4), q, t, ninv)),
+                        lambda: cuda.mul_inverse_batch(ntts, P(o), P(d4), P(e4), c, 1)),
+        "chain mul 1": (limbs(lambda i, q, t, *_: fwd(oracle.mul(back[i], m2[i], q, 2), q, t)),
+                        lambda: cuda.chain_mul_batch(ntts, P(o), P(d2), P(e2), c, 2, 1)),
+        "chain fma 4": (limbs(lambda i, q, t, *_: fwd(oracle.fma(back[i], sc[i % L], m2[i], q, 2), q, t, 4)),
+                        lambda: cuda.chain_fma_batch(ntts, P(o), P(d2), sc, P(e2), c, 2, 4)),
+        "product 1": (limbs(lambda i, q, f, t, ninv: inv(prod[i], q, t, ninv)),
+                      lambda: cuda.product_batch(ntts, P(o), P(d4), P(e4), c, 4, 1)),
+        "product 2": (limbs(lambda i, q, f, t, ninv: inv(prod[i], q, t, ninv, 2)),
+                      lambda: cuda.product_batch(ntts, P(o), P(d4), P(e4), c, 4, 2)),
+    }
+    ran = dict.fromkeys(ops, 0)
+    try:
+        for plan in plans(logn):
+            cuda.plan_set(False, logn, plan)
+            try:
+                cuda.plan_set(True, logn, plan[::-1])  # its tiles may not fit the inverse's strides
+            except cuda.AxhelError:
+                cuda.plan_set(True, logn, [])
+            for name, (want, run) in ops.items():
+                o.fill_(-1)
+                try:
+                    run()
+                except cuda.AxhelError:
+                    # a chain or product runs the inverse plan's passes both ways round
+                    assert name[:7] in ("chain m", "chain f", "product"), name
+                    continue
+                ran[name] += 1
+                assert torch.equal(o, want), f"{name} under {plan}"
+    finally:
+        cuda.plan_set(False, logn, [])
+        cuda.plan_set(True, logn, [])
+    assert min(ran.values()) >= 1, ran
