@@ -737,7 +737,7 @@ axhel_status_t product(const axhel_ntt_t* ntts, uint64_t n_ntts, uint64_t* resul
     c.pass.dst = result;
     c.pass.s0 = 0;
     c.pass.tg = (uint32_t)fc.tg;
-    c.pass.flags = relax_in | relax_out |
+    c.pass.flags = relax_in | relax_out | (fp_any(ntts, n_ntts) ? (uint32_t)kFpLimbs : 0u) |
                    (inv.npass == 1 ? ((uint32_t)kLastPass | (out_f != 2 ? (uint32_t)kPostNorm : 0u)) : 0u);
     c.operand = vec;
     c.op = kChainMul;

@@ -53,6 +53,7 @@ enum PassFlags : uint32_t {
     kRelaxOut = 32u,     // the transform's output is normalized: its stages may work on other representatives
     kRelaxIn = 64u,      // fused chain / product passes: likewise the transform ahead of the op
     kLazyFp = 128u,      // lazy forward passes may run in FP64 where the modulus allows
+    kFpLimbs = 256u,     // product passes: some moduli have the FP64 form
 };
 
 // Geometry of one pass: stages [s0, s0 + lg) of an N = 2^logn transform, on

@@ -39,16 +39,25 @@ cudaError_t ensure_smem(Fn fn, FnKind kind, bool relax, int column, bool row, co
 }
 
 // Whether a launch's limbs run two per thread, pairs of the batch's groups of
-// nctx limbs (one per modulus); a last group without a partner costs as much
-// as a pair, so a few odd groups stay single.
+// nctx limbs (one per modulus).  A limb without a partner costs an FP64 pass as
+// much as a pair (41 limbs of 40 45-bit moduli, N = 2^16: lazy product 102 us
+// as pairs, 59.4 single), so batches with more than a seventh of them stay single.
+// The integer product passes run a pair's limbs in turn and do not have that
+// cost (40 limbs of 24 55-bit moduli 3-4 % faster as pairs).
 bool pairs(FnKind kind, bool relax, const PassCfg& c, const PassArgs& a)
 {
     if (kind == kFnFwd && !relax) return false;  // the lazy forms: 333 against 320 us for 768 limbs of 2^16
     if (!relaxed_compiled(c.lg, c.lr) || (smem_bytes(c) << 1) > 227 * 1024) return false;
-    const uint64_t groups = (a.count + a.nctx - 1) / a.nctx;
-    if (groups < 2 || ((groups & 1) && groups < 7)) return false;
-    return ((a.count << a.logn) >> (c.lr + 1)) >= (uint64_t)sm_count() * kPairThreadsPerSm;
+    if (((a.count << a.logn) >> (c.lr + 1)) < (uint64_t)sm_count() * kPairThreadsPerSm) return false;
+    const uint64_t groups = (a.count + a.nctx - 1) / a.nctx, paired = 2 * a.nctx * ((groups + 1) / 2);
+    if (kind == kFnProduct && !(a.flags & kFpLimbs)) return groups >= 7 || groups % 2 == 0;
+    return 7 * paired <= 8 * a.count;
 }
+
+PassArgs& pass_of(PassArgs& a) { return a; }
+PassArgs& pass_of(ChainArgs& a) { return a.pass; }
+void copy_scalar(PassArgs&, uint64_t, uint64_t) {}
+void copy_scalar(ChainArgs& a, uint64_t to, uint64_t from) { a.scalar[to] = a.scalar[from]; }
 
 // Launches a pass over its limbs; `pass` is the PassArgs inside the kernel's
 // argument struct `args`.
@@ -64,12 +73,32 @@ cudaError_t launch_tiles(const FnTable<void (*)(const Args)>& t, FnKind kind, bo
     const cudaError_t e = ensure_smem(fn, kind, relax, plain ? kSmemPlain : pair, row, c);
     if (e != cudaSuccess) return e;
     const uint64_t per_limb = (1ull << (pass.logn - c.lg)) / c.tg;
-    const uint64_t moduli = pass.count < pass.nctx ? pass.count : pass.nctx;
-    const uint64_t groups = (pass.count + moduli - 1) / moduli;
-    const uint64_t gx = ((groups + pair) >> pair) * per_limb;
     if (pass.count * per_limb > 0x7fffffffull) return cudaErrorInvalidValue;
+    const unsigned threads = (unsigned)c.tg << (c.lg - c.lr);
     count_launch();
-    fn<<<dim3((unsigned)gx, (unsigned)moduli), (unsigned)c.tg << (c.lg - c.lr), smem_bytes(c) << pair, s>>>(args);
+    // A last group that holds only some of the moduli: the CTAs of its missing
+    // limbs would lie between the others and leave SMs idle.  Few limbs are
+    // launched as one group, each with its own context (N = 2^16, 55 bits, us:
+    // 9 limbs of 8 moduli forward 13.7 to 10.7, product 30.6 to 22.1; 32 of 24
+    // 28.9 to 25.9, 67.9 to 64.1); otherwise the groups go to blockIdx.z, which puts those CTAs last
+    // (300 limbs of 24 moduli of 2^13: 28.2 to 26.4, 60.2 to 56.0).
+    const uint64_t moduli = pass.count < pass.nctx ? pass.count : pass.nctx;
+    const bool partial = pass.count % moduli != 0;
+    if (partial && !pair && pass.count <= (uint64_t)kMaxInlineMods) {
+        Args one = args;
+        PassArgs& p = pass_of(one);
+        p.nctx = (uint32_t)pass.count;
+        for (uint64_t i = moduli; i < pass.count; ++i) {
+            p.ctx[i] = p.ctx[i - moduli];
+            copy_scalar(one, i, i - moduli);
+        }
+        fn<<<dim3((unsigned)per_limb, p.nctx), threads, smem_bytes(c), s>>>(one);
+        return cudaGetLastError();
+    }
+    const uint64_t groups = (pass.count + moduli - 1) / moduli, gs = (groups + pair) >> pair;
+    const bool in_z = partial && gs <= 65535;
+    const dim3 grid((unsigned)(in_z ? per_limb : gs * per_limb), (unsigned)moduli, in_z ? (unsigned)gs : 1);
+    fn<<<grid, threads, smem_bytes(c) << pair, s>>>(args);
     return cudaGetLastError();
 }
 

@@ -82,6 +82,43 @@ def test_forms_match_oracle(cuda, oracle, n, polys):
             np.testing.assert_array_equal(got[i], expect(i), err_msg=f"{name}: limb {i}, q of {qs[i].bit_length()} bits")
 
 
+# The last group of limbs holds some of the moduli only: few limbs (up to 64), more,
+# and enough for two limbs per thread, with and without partners for most.
+@pytest.mark.parametrize("n,counts", [(4096, (66, 71, 606, 1008)), (16384, (8, 13, 33, 64, 65, 160)), (65536, (8, 13, 39)),
+                                      (131072, (9,))])
+def test_partial_last_group(cuda, oracle, n, counts):
+    mods = limit_moduli(oracle, n)
+    L, top = len(mods), max(counts)
+    ntts = cuda.NTT.create_many([(n, q, psi) for q, psi in mods])
+    tabs = [oracle.tables(n, q, psi) for q, psi in mods]
+    rng = np.random.default_rng(n)
+    qs = [mods[i % L][0] for i in range(top)]
+    x, m = inputs(rng, n, [2 * q for q in qs]), inputs(rng, n, [2 * q for q in qs])
+    sc = [(2 * q) // 3 for q, _ in mods]
+    d, e, o = dev(x), dev(m), dev_empty(top * n)
+    fwd = lambda i, v, f=1: oracle.forward(v, qs[i], tabs[i % L][0], 1, f)
+    inv = lambda i, v, f=1: oracle.inverse(v, qs[i], tabs[i % L][1], tabs[i % L][2], 2, f)
+    ops = {
+        "forward 1": (lambda c: cuda.forward_batch(ntts, ptr(o), ptr(d), c, 2, 1), lambda i: fwd(i, x[i])),
+        "forward 4": (lambda c: cuda.forward_batch(ntts, ptr(o), ptr(d), c, 2, 4), lambda i: fwd(i, x[i], 4)),
+        "inverse 1": (lambda c: cuda.inverse_batch(ntts, ptr(o), ptr(d), c, 2, 1), lambda i: inv(i, x[i])),
+        "chain fma 1": (lambda c: cuda.chain_fma_batch(ntts, ptr(o), ptr(d), sc, ptr(e), c, 2, 1),
+                        lambda i: fwd(i, oracle.fma(inv(i, x[i], 2), sc[i % L], m[i], qs[i], 2))),
+        "chain fma 4": (lambda c: cuda.chain_fma_batch(ntts, ptr(o), ptr(d), sc, 0, c, 2, 4),
+                        lambda i: fwd(i, oracle.fma(inv(i, x[i], 2), sc[i % L], None, qs[i], 2), 4)),
+        "product 1": (lambda c: cuda.product_batch(ntts, ptr(o), ptr(d), ptr(e), c, 4, 1),
+                      lambda i: inv(i, oracle.mul(fwd(i, x[i], 4), m[i], qs[i], 4))),
+    }
+    for name, (run, expect) in ops.items():
+        want = np.stack([expect(i) for i in range(top)])
+        for c in counts:
+            o.fill_(-1)
+            run(c)
+            got = host(o).reshape(top, n)
+            np.testing.assert_array_equal(got[:c], want[:c], err_msg=f"{name}, {c} limbs")
+            assert (got[c:] == np.uint64(2 ** 64 - 1)).all(), f"{name}, {c} limbs: written past the last"
+
+
 @pytest.mark.parametrize("bits", [50, 59])
 def test_in_place_and_unaligned(cuda, oracle, bits):
     """In place, and at 8- and 16-byte aligned addresses (the wide accesses fall back)."""
