@@ -443,10 +443,17 @@ axhel_status_t collect(const axhel_ntt_t* ntts, uint64_t n_ntts, PassArgs& a, ui
 // against 10.0, 768 limbs of 2^16 499 against 549).
 constexpr uint64_t kLazyFpWords = 3ull << 17;
 
-// A fused chain or product of fewer residues without FP64 moduli keeps the
-// reference's integer butterflies: in a wave that leaves the GPU half empty
-// the relaxed ones' range reductions only lengthen the chain (one limb of
-// N = 2^17: product 16.5 against 15.4 us; 40 limbs of 2^15 32.4 against 41.8).
+// Fused chains and products.  In a wave that leaves the GPU half empty the
+// relaxed integer butterflies' range reductions only lengthen the chain, and one
+// limb with them is as long as all.  Up to kFpAllWords residues the forms are
+// taken if every modulus has the FP64 one, up to kRelaxIntWords if some have.
+// Us, reference's butterflies then the forms: 55-bit moduli, 2^17 residues (one
+// limb of N = 2^17) product 13.1 and 16.2; 2^18 (8 limbs of 2^15) chain 14.7 and
+// 16.4; 2^19 22.7 and 21.8 (64 of 2^13 20.3 and 19.2); 2^20 36.1 and 35.0; lazy
+// outputs 14.5 and 16.9, 22.5 and 22.7, 35.6 and 35.8.  Half the moduli of 45
+// bits: 2^18 chain 15.2 and 16.4, lazy 15.1 and 17.8; 3 x 2^17 (12 limbs of 2^15)
+// 18.8 and 17.9, 18.6 and 19.1.
+constexpr uint64_t kFpAllWords = 1ull << 18;
 constexpr uint64_t kRelaxIntWords = 1ull << 19;
 
 uint64_t fp_moduli(const axhel_ntt_t* ntts, uint64_t n_ntts)
@@ -455,7 +462,6 @@ uint64_t fp_moduli(const axhel_ntt_t* ntts, uint64_t n_ntts)
     for (uint64_t i = 0; i < n_ntts; ++i) k += !ntts[i]->external && ntts[i]->q < kFpModulusEnd;
     return k;
 }
-bool fp_any(const axhel_ntt_t* ntts, uint64_t n_ntts) { return fp_moduli(ntts, n_ntts) != 0; }
 
 // Whether any modulus has another form than the reference's butterflies: the
 // others keep the plan that was tuned for those (16 registers per thread in the
@@ -468,6 +474,15 @@ bool any_form(const axhel_ntt_t* ntts, uint64_t n_ntts)
     for (uint64_t i = 0; i < n_ntts; ++i)
         if (has_forms(ntts[i])) return true;
     return false;
+}
+
+// Whether the inner halves of a fused chain or product (and, with a normalized
+// output, its outer ones) take the forms the moduli have.
+bool fused_forms(const axhel_ntt_t* ntts, uint64_t n_ntts, uint32_t logn, uint64_t count)
+{
+    const uint64_t words = count << logn;
+    if (words >= kRelaxIntWords) return any_form(ntts, n_ntts);
+    return fp_moduli(ntts, n_ntts) >= (words > kFpAllWords ? 1 : n_ntts);
 }
 
 // Whether a quarter of the moduli or more have FP64 forms.
@@ -614,8 +629,7 @@ axhel_status_t chain(const axhel_ntt_t* ntts, uint64_t n_ntts, uint64_t* result,
         inv = NttPlan{1, {PassCfg{(int)logn, logn < 3 ? (int)logn : 3, 1}}};
     // the op takes any representative of the inverse's output, and a
     // normalized forward may work on any
-    const bool relaxable =
-        ((count << logn) >= kRelaxIntWords ? any_form(ntts, n_ntts) : fp_any(ntts, n_ntts)) && plan_relax(true, logn, inv);
+    const bool relaxable = fused_forms(ntts, n_ntts, logn, count) && plan_relax(true, logn, inv);
     const uint32_t relax_in = relaxable ? (uint32_t)kRelaxIn : 0u;
     const uint32_t relax_out = relaxable && out_f != 4 ? (uint32_t)kRelaxOut : 0u;
     // forward passes after the fused one: the inverse's earlier passes, reversed
@@ -709,8 +723,7 @@ axhel_status_t product(const axhel_ntt_t* ntts, uint64_t n_ntts, uint64_t* resul
     cudaStream_t s = S(stream);
     // the MulMod takes any representative of the forward's output, and a
     // normalized inverse may work on any
-    const bool relaxable =
-        ((count << logn) >= kRelaxIntWords ? any_form(ntts, n_ntts) : fp_any(ntts, n_ntts)) && plan_relax(true, logn, inv);
+    const bool relaxable = fused_forms(ntts, n_ntts, logn, count) && plan_relax(true, logn, inv);
     const uint32_t relax_in = relaxable ? (uint32_t)kRelaxIn : 0u;
     const uint32_t relax_out = relaxable && out_f != 2 ? (uint32_t)kRelaxOut : 0u;
     // fused: forward last pass -> MulMod -> inverse first pass (register depth 3:
@@ -737,7 +750,7 @@ axhel_status_t product(const axhel_ntt_t* ntts, uint64_t n_ntts, uint64_t* resul
     c.pass.dst = result;
     c.pass.s0 = 0;
     c.pass.tg = (uint32_t)fc.tg;
-    c.pass.flags = relax_in | relax_out | (fp_any(ntts, n_ntts) ? (uint32_t)kFpLimbs : 0u) |
+    c.pass.flags = relax_in | relax_out | (fp_moduli(ntts, n_ntts) != 0 ? (uint32_t)kFpLimbs : 0u) |
                    (inv.npass == 1 ? ((uint32_t)kLastPass | (out_f != 2 ? (uint32_t)kPostNorm : 0u)) : 0u);
     c.operand = vec;
     c.op = kChainMul;

@@ -80,8 +80,9 @@ cudaError_t launch_tiles(const FnTable<void (*)(const Args)>& t, FnKind kind, bo
     // limbs would lie between the others and leave SMs idle.  Few limbs are
     // launched as one group, each with its own context (N = 2^16, 55 bits, us:
     // 9 limbs of 8 moduli forward 13.7 to 10.7, product 30.6 to 22.1; 32 of 24
-    // 28.9 to 25.9, 67.9 to 64.1); otherwise the groups go to blockIdx.z, which puts those CTAs last
-    // (300 limbs of 24 moduli of 2^13: 28.2 to 26.4, 60.2 to 56.0).
+    // 28.9 to 25.9, 67.9 to 64.1); otherwise the groups go to blockIdx.z, which
+    // puts those CTAs last (300 limbs of 24 moduli of 2^13: 28.2 to 26.4, 60.2 to
+    // 56.0).
     const uint64_t moduli = pass.count < pass.nctx ? pass.count : pass.nctx;
     const bool partial = pass.count % moduli != 0;
     if (partial && !pair && pass.count <= (uint64_t)kMaxInlineMods) {
