@@ -493,15 +493,18 @@ bool fp_share(const axhel_ntt_t* ntts, uint64_t n_ntts) { return 4 * fp_moduli(n
 // FP64 are as fast or faster although they may cost two launches more: from
 // 2^18 residues on, which the shipped limits reach at 64 limbs of N = 2^12 and
 // 32 of 2^13.  Calls one after the other, us, cluster form then passes: there
-// chains 12.3 and 10.3, 16.4 and 14.9 (lazy output 12.3 and 12.3, 16.4 and
-// 16.4), products 12.2 and 10.3, 14.4 and 14.4; at 31 limbs of 2^13 12.4 and
-// 15.7, at 4 of 2^15 14.5 and 14.9.  A cluster shape set by the caller is used.
+// chains 12.3 and 10.3, 16.4 and 14.9, products 12.2 and 10.3, 14.4 and 14.4; at
+// 31 limbs of 2^13 12.4 and 15.7, at 4 of 2^15 14.5 and 14.9.  Lazy outputs stay
+// in the cluster form at 2^12, where the passes are one of a CTA per limb (on the
+// device chain 9.6 and 10.8, product 10.0 and 11.0; of 2^13 14.3 and 12.0, 13.7
+// and 11.1).  A cluster shape set by the caller is used.
 // Not for single transforms: one limb of 2^15 takes 5.2 us as two passes
 // against 7.3 on the device, but calls one after the other are bound by the
 // second launch (8 limbs of 2^14 8.3 and 10.4).
-bool fp_passes_win(ClusterKind kind, const axhel_ntt_t* ntts, uint64_t n_ntts, uint32_t logn, uint64_t count)
+bool fp_passes_win(ClusterKind kind, const axhel_ntt_t* ntts, uint64_t n_ntts, uint32_t logn, uint64_t count,
+                   bool norm)
 {
-    return (count << logn) >= (1ull << 18) && !cluster_plan_overridden(kind, logn) &&
+    return (count << logn) >= (1ull << 18) && (norm || logn > 12) && !cluster_plan_overridden(kind, logn) &&
            fp_moduli(ntts, n_ntts) == n_ntts;
 }
 
@@ -611,7 +614,7 @@ axhel_status_t chain(const axhel_ntt_t* ntts, uint64_t n_ntts, uint64_t* result,
     // a few limbs: the whole chain in one launch, one cluster per limb
     ClusterCfg cc;
     if (!plan_overridden(true, logn) && cluster_plan(kClusterChain, logn, count, &cc) &&
-        (vec_in_result || !fp_passes_win(kClusterChain, ntts, n_ntts, logn, count))) {
+        (vec_in_result || !fp_passes_win(kClusterChain, ntts, n_ntts, logn, count, out_f != 4))) {
         c.pass.src = operand;
         c.pass.dst = result;
         c.pass.flags = (in_f == 4 ? (uint32_t)kPreCsub2q : 0u) | (out_f != 4 ? (uint32_t)kPostNorm : 0u);
@@ -708,7 +711,7 @@ axhel_status_t product(const axhel_ntt_t* ntts, uint64_t n_ntts, uint64_t* resul
     // a few limbs: the whole product in one launch, one cluster per limb
     ClusterCfg cc;
     if (!plan_overridden(true, logn) && cluster_plan(kClusterProduct, logn, count, &cc) &&
-        !fp_passes_win(kClusterProduct, ntts, n_ntts, logn, count)) {
+        !fp_passes_win(kClusterProduct, ntts, n_ntts, logn, count, out_f != 2)) {
         c.pass.src = operand;
         c.pass.dst = result;
         c.pass.flags = out_f != 2 ? (uint32_t)kPostNorm : 0u;

@@ -454,7 +454,8 @@ axhel_status_t axhel_cuda_plan_get(int inverse, uint32_t log_degree, uint64_t co
  * groups); `lr` register stages.  Used for 2^10 <= N <= 2^17 and count <=
  * max_limbs; max_limbs == 0 turns it off for (kind, log2 N), lga == 0
  * restores the built-in choice (with which kinds 2 and 3 take the passes from
- * 2^18 residues on if all moduli are below 2^50).  A pass plan set by
+ * 2^18 residues on if all moduli are below 2^50, lazy outputs only above
+ * N = 2^12).  A pass plan set by
  * axhel_cuda_plan_set for the same degree (the inverse plan, for kinds 2 and
  * 3) takes precedence.  Every choice computes the same bits. */
 axhel_status_t axhel_cuda_cluster_plan_set(int kind, uint32_t log_degree, uint32_t lga, uint32_t lr,

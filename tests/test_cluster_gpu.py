@@ -273,3 +273,31 @@ def test_cluster_shape_set_by_hand_is_used(cuda, oracle, kind):
         cuda.cluster_plan_set(k, logn)
     assert names == [f"ntt_{kind}_cluster lgr=6 lr=2 c=8"]
     np.testing.assert_array_equal(got, want)
+
+
+@pytest.mark.parametrize("kind,lazy", [("chain", 4), ("product", 2)])
+def test_lazy_fused_calls_keep_the_cluster_form(cuda, oracle, kind, lazy):
+    """64 limbs of N = 2^12 below 2^50: normalized outputs take the FP64 pass, lazy ones the cluster."""
+    n, count = 4096, 64
+    q = oracle.find_ntt_prime_near(n, 45, 1, 1)
+    psi = oracle.find_primitive_root(n, q)
+    t = cuda.NTT(n, q, psi)
+    fwd, inv, ninv = oracle.tables(n, q, psi)
+    rng = np.random.default_rng(64)
+    x, m = (rng.integers(0, q, (count, n), dtype=np.uint64) for _ in range(2))
+    d, e, o = dev(x), dev(m), dev_empty(count * n)
+    f = cuda.chain_mul_batch if kind == "chain" else cuda.product_batch
+    for out_f, cluster in ((1, False), (lazy, True)):
+        cuda.profile_enable(True)
+        cuda.profile_report()
+        f([t], ptr(o), ptr(d), ptr(e), count, 1, out_f)
+        names = list(cuda.profile_report())
+        cuda.profile_enable(False)
+        assert ["cluster" in s for s in names] == [cluster], names
+        got = host(o).reshape(count, n)
+        for i in (0, count - 1):
+            if kind == "chain":
+                want = oracle.forward(oracle.mul(oracle.inverse(x[i], q, inv, ninv, 1, 2), m[i], q, 2), q, fwd, 1, out_f)
+            else:
+                want = oracle.inverse(oracle.mul(oracle.forward(x[i], q, fwd, 1, 4), m[i], q, 4), q, inv, ninv, 2, out_f)
+            np.testing.assert_array_equal(got[i], want)
