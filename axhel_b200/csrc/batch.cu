@@ -671,16 +671,25 @@ axhel_status_t batch_build(const axhel_job_t* jobs, uint64_t n_jobs, unsigned ch
         ent_cls[k] = pc.chain ? kClsChain : (pc.inv ? kClsInv : kClsFwd);
         ent_lg[k] = pc.lg;
     }
-    // the arithmetics of every entry, from its job's: a chain's inverse feeds
+    // The arithmetics of every entry, from its job's: a chain's inverse feeds
     // a MulMod / FMAMod, which takes any representative; lazy forwards run in
-    // FP64 where a quarter of the moduli or more have it; jobs without such
-    // moduli in the kernels of the reference's butterflies
+    // FP64 where a quarter of the moduli or more have it.  Jobs with fewer FP64
+    // moduli take the kernels of the reference's butterflies up to
+    // kRelaxJobWords residues: kernels by form split a phase into more launches
+    // (a half more for wide moduli), which the relaxed integers do not earn back.
+    // Batches of jobs of 50-58 bits, against the reference's butterflies
+    // everywhere: with the forms for all 0.90 of the speed (24 jobs of 1-24
+    // limbs, N = 2^12..2^16), 0.97 (64), 1.13 (4 of 64-192 limbs); from 2^21
+    // residues on 1.01, 1.07 and 1.14; from 2^19 1.00, 1.03 and 1.13; for none
+    // 1.01, 1.07 and 1.13 (one such large job 1.07, 1.05, 1.07 and 1.03).
+    constexpr uint64_t kRelaxJobWords = 1ull << 21;
     std::vector<uint32_t> ent_flags(ent.size(), 0), ent_forms(ent.size(), kFormsExact);
     for (size_t k = 0; k < ent.size(); ++k) {
         const BatchJob& b = bj[ent[k].job];
         if (b.kind >= kJobAdd || n_form[ent[k].job] == 0) continue;
         const bool chain = b.kind == kJobChainMul || b.kind == kJobChainFma, inverse = ent_cls[k] == kClsInv;
         const bool lazy_fp = 4 * n_fp[ent[k].job] >= b.nmods;
+        if (!lazy_fp && (b.count << b.logn) < kRelaxJobWords) continue;
         uint32_t& f = ent_flags[k];
         if (chain && ent_cls[k] == kClsChain) f |= kRelaxIn;
         if ((chain && inverse) || b.norm) f |= kRelaxOut;

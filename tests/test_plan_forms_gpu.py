@@ -90,6 +90,26 @@ def test_batches_of_exact_moduli(cuda, oracle, phased):
     b.close()
 
 
+def test_small_jobs_of_wide_moduli_share_their_launches(cuda, oracle):
+    """Small jobs without FP64 moduli, lazy and normalized outputs: one launch per
+    phase, class and pass width, as for the reference's butterflies."""
+    n, count = 4096, 3
+    q, (fwd, inv, ninv), t = make(cuda, oracle, n, 55, False)
+    rng = np.random.default_rng(55)
+    x = [rng.integers(0, q, (count, n), dtype=np.uint64) for _ in range(4)]
+    d, outs = [dev(v) for v in x], [dev_empty(count * n) for _ in x]
+    b = cuda.Batch([dict(kind=cuda.JOB_FORWARD, ntts=[t], count=count, result=ptr(o), operand=ptr(i), in_f=1,
+                         out_f=(1, 4)[j % 2]) for j, (i, o) in enumerate(zip(d, outs))])
+    b.launch(phased=True)
+    before = cuda.launch_count()
+    b.launch(phased=True)
+    assert cuda.launch_count() - before == 2
+    for j, o in enumerate(outs):
+        want = np.stack([oracle.forward(v, q, fwd, 1, (1, 4)[j % 2]) for v in x[j]])
+        np.testing.assert_array_equal(host(o).reshape(count, n), want)
+    b.close()
+
+
 # 16 registers per thread (the reference's butterflies), and 8 with tiles wider
 # than the relaxed modes' own
 @pytest.mark.parametrize("bits", [45, 55])
