@@ -104,10 +104,12 @@ __device__ __forceinline__ void st_words4(uint64_t* p, const uint64_t (&x)[4])
 // pipe per warp and element) and the loads have to overlap across warps, so
 // what counts is warps in flight: one 32-byte vector per operand and thread,
 // 40-48 registers, twice the CTAs, against four 16-byte ones at 64-80
-// registers in eltwise_vec_kernel.  MulMod, 59-bit modulus: 2^20 elements 8.4
-// to 6.4 us, 2^22 20.7 to 18.8, 2^24 72.1 to 64.1 (6.28 TB/s); FMAMod 8.4 to
-// 6.8, 22.8 to 19.4, 76.1 to 65.9.  Operands that share their offset from a
-// 32-byte boundary start with `head` single elements and end with a tail.
+// registers in eltwise_vec_kernel.  MulMod<4>, 59-bit modulus, calls one after
+// the other: 2^20 elements 8.8 to 7.1 us, 2^22 21.1 to 18.9, 2^24 76.1 to 65.3;
+// factor 1 7.1 to 6.5, 17.6 to 14.9, 64.5 to 63.2 (6.37 TB/s); FMAMod<4> 8.7 to
+// 7.7, 23.0 to 21.0, 79.7 to 72.1; factor 1 7.3 to 6.6, 18.9 to 16.8, 65.2 to
+// 63.9.  Operands that share their offset from a 32-byte boundary start with
+// `head` single elements and end with a tail.
 template <class Op, bool HAS_B>
 __global__ void __launch_bounds__(256) eltwise_product_kernel(uint64_t* r, const uint64_t* a, const uint64_t* b,
                                                               uint64_t n, uint32_t head, const Op op)
@@ -140,9 +142,14 @@ static cudaError_t run(uint64_t* r, const uint64_t* a, const uint64_t* b, uint64
         const uintptr_t at = reinterpret_cast<uintptr_t>(r);
         const uintptr_t differ = (at ^ reinterpret_cast<uintptr_t>(a)) |
                                  (HAS_B ? at ^ reinterpret_cast<uintptr_t>(b) : 0);
-        if ((differ & 31) == 0 && (at & 7) == 0) {
-            uint64_t head = (32 - at % 32) % 32 / 8;
-            if (head > n) head = n;
+        const uint64_t head = (32 - at % 32) % 32 / 8;
+        // A head is a second, dependent round of loads in the first CTA: small
+        // calls with one take the kernels below (device us: 8-byte aligned
+        // operands, 2^16 elements 1.81 there and 2.32 here, 2^18.5 2.85 and 3.09,
+        // 2^19 3.52 and 3.56, 2^20 5.53 and 5.16; 16-byte aligned ones 2^8 1.82
+        // and 2.14, 2^10 2.27 and 2.35, 2^12 2.84 and 2.34).
+        const uint64_t least = head == 0 ? 0 : ((at & 15) ? 1u << 19 : 1u << 11);
+        if ((differ & 31) == 0 && (at & 7) == 0 && n >= least) {
             uint64_t blocks = ((n - head) / 4 + threads - 1) / threads;
             const uint64_t cap = (uint64_t)sm_count() * 16;
             if (blocks > cap) blocks = cap;
@@ -372,21 +379,28 @@ cudaError_t tensor_product(uint64_t* r0, uint64_t* r1, uint64_t* r2, const uint6
         a.m[i].fq = (double)moduli[i];
         a.m[i].fqi = 1.0 / a.m[i].fq;
     }
+    bool fp = false;
+    for (uint64_t i = 0; i < nmod; ++i) fp |= a.m[i].fp != 0;
     if (n == 0 || count == 0) return cudaSuccess;
     const int threads = 256;
     uint64_t bx = (n / 2 + threads - 1) / threads;
-    // 64 CTAs per SM in total, at least one per limb (8: 305 us, 64: 293, one
-    // chunk per CTA: 326, on the shape above)
-    uint64_t want = ((uint64_t)sm_count() * 64 + count - 1) / count;
+    // CTAs per SM in total, at least one per limb: 64 with FP64 moduli (8: 305
+    // us, 64: 293, one chunk per CTA: 326, on the shape above); 16 without, in
+    // a power of two of CTAs per limb, so that they share its chunks evenly
+    // (59 bits, against 8: 32 limbs of N = 2^15 12.0 to 10.7 us, 64 of 2^17 83.5
+    // to 78.8; 3 CTAs for the 8 chunks of 1024 limbs of 2^12 41.0 to 42.7, 2 41.0).
+    uint64_t want = ((uint64_t)sm_count() * (fp ? 64 : 16) + count - 1) / count;
     if (want < 1) want = 1;
+    if (!fp)
+        while (want & (want - 1)) want &= want - 1;
     if (bx > want) bx = want;
     const dim3 grid((unsigned)bx, (unsigned)count);
     count_launch();
     ProfScope prof(s, "tensor_product f=%d", (int)factor);
     switch (factor) {
-    case 1: tensor_product_kernel<1><<<grid, threads, 0, s>>>(a); break;
-    case 2: tensor_product_kernel<2><<<grid, threads, 0, s>>>(a); break;
-    case 4: tensor_product_kernel<4><<<grid, threads, 0, s>>>(a); break;
+    case 1: (fp ? tensor_product_kernel<1, true> : tensor_product_kernel<1, false>)<<<grid, threads, 0, s>>>(a); break;
+    case 2: (fp ? tensor_product_kernel<2, true> : tensor_product_kernel<2, false>)<<<grid, threads, 0, s>>>(a); break;
+    case 4: (fp ? tensor_product_kernel<4, true> : tensor_product_kernel<4, false>)<<<grid, threads, 0, s>>>(a); break;
     default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();

@@ -290,3 +290,31 @@ def test_product_alignments(cuda, oracle, n, offsets):
         got = host(o)
         np.testing.assert_array_equal(got[offsets[0]:offsets[0] + n], exp, err_msg=name)
         assert not got[:offsets[0]].any() and not got[offsets[0] + n:].any(), f"{name}: wrote outside"
+
+
+# MulMod / FMAMod around the sizes from which operands off a 32-byte boundary take
+# the 32-byte kernel: 16-byte aligned from 2^11 elements, 8-byte aligned from 2^19.
+@pytest.mark.parametrize("words,least", [(0, 1), (1, 1 << 19), (2, 1 << 11), (3, 1 << 19)])
+def test_product_kernel_choice(cuda, oracle, words, least):
+    q = (1 << 59) - 55
+    rng = np.random.default_rng(words)
+    for n in sorted({1, 5, least - 1, least, least + 3}):
+        if n < 1:
+            continue
+        a, b = (rng.integers(0, q, n, dtype=np.uint64) for _ in range(2))
+        da, db = (dev(np.concatenate([np.zeros(words, np.uint64), v])) for v in (a, b))
+        o = dev_empty(n + words + 1, fill=7)
+        for run, want in ((lambda: cuda.mul(ptr(o) + 8 * words, ptr(da) + 8 * words, ptr(db) + 8 * words, n, q, 1),
+                           oracle.mul(a, b, q, 1)),
+                          (lambda: cuda.fma(ptr(o) + 8 * words, ptr(da) + 8 * words, q // 3, ptr(db) + 8 * words, n, q, 1),
+                           oracle.fma(a, q // 3, b, q, 1))):
+            cuda.profile_enable(True)
+            cuda.profile_report()
+            run()
+            names = list(cuda.profile_report())
+            cuda.profile_enable(False)
+            got = host(o)
+            np.testing.assert_array_equal(got[words:words + n], want, err_msg=f"n={n}")
+            assert got[words + n] == 7 and (got[:words] == 7).all()
+            if words % 2:
+                assert names[0].endswith("_unaligned") == (n < least), (n, names)
