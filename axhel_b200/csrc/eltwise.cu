@@ -295,7 +295,9 @@ struct TensorArgs {
 // products are about 180 clocks of the multiply pipe per warp and element, of
 // the 300 or so that its bytes take.  Moduli below 2^50 take about 40 FP64
 // instructions of two clocks instead.  64 pairs x 16 limbs (40-55 bits) of
-// N = 2^15: factor 1 305 to 285 us (6.6 TB/s), factor 4 360 to 288.
+// N = 2^15: factor 1 305 to 285 us (6.6 TB/s), factor 4 360 to 288.  Calls
+// without such moduli run a kernel without that form (59 bits, 1024 limbs of
+// N = 2^12: factor 1 48.8 us with it, 41.0 without).
 template <int F>
 __device__ __forceinline__ void tensor_fp(uint64_t c0, uint64_t c1, uint64_t d0, uint64_t d1, uint64_t& r0,
                                           uint64_t& r1, uint64_t& r2, double q, double qi)
@@ -315,7 +317,7 @@ __device__ __forceinline__ void tensor_fp(uint64_t c0, uint64_t c1, uint64_t d0,
     r1 = fp_canon(fp_reduce(__dadd_rn(__dadd_rn(p1, -p0), -p2), q, qi), q);
 }
 
-template <int F>
+template <int F, bool FP>
 __global__ void __launch_bounds__(256) tensor_product_kernel(const __grid_constant__ TensorArgs a)
 {
     // grid: x = chunks of one limb, y = limb.  Two elements per thread step.
@@ -346,7 +348,7 @@ __global__ void __launch_bounds__(256) tensor_product_kernel(const __grid_consta
         const ulonglong2 y0 = *reinterpret_cast<const ulonglong2*>(a.d0 + off + e);
         const ulonglong2 y1 = *reinterpret_cast<const ulonglong2*>(a.d1 + off + e);
         uint64_t r[2][3];
-        if (mc.fp) {
+        if (FP && mc.fp) {
             tensor_fp<F>(x0.x, x1.x, y0.x, y1.x, r[0][0], r[0][1], r[0][2], mc.fq, mc.fqi);
             tensor_fp<F>(x0.y, x1.y, y0.y, y1.y, r[1][0], r[1][1], r[1][2], mc.fq, mc.fqi);
         } else {

@@ -157,3 +157,20 @@ def test_tensor_forms(cuda, oracle, factor):
         exp = (mul(c0, d0), oracle.add(mul(c0, d1), mul(c1, d0), q), mul(c1, d1))
         for k in range(3):
             np.testing.assert_array_equal(got[k][i], exp[k], err_msg=f"limb {i} output {k} q={q}")
+
+
+@pytest.mark.parametrize("n,count", [(2, 1), (514, 3), (4096, 40), (2048, 1024), (32768, 9)])
+def test_tensor_without_fp64_moduli(cuda, oracle, n, count):
+    qs = [(1 << 50) + 55, (1 << 61) + 15]
+    rng = np.random.default_rng(n)
+    x = [np.stack([rng.integers(0, 2 * qs[i % 2], n, dtype=np.uint64) for i in range(count)]) for _ in range(4)]
+    d = [dev(v) for v in x]
+    r = [dev_empty(count * n) for _ in range(3)]
+    cuda.tensor_product(*[ptr(t) for t in (*r, *d)], n, count, qs, 2)
+    got = [host(t).reshape(count, n) for t in r]
+    for i in sorted({0, 1, count // 2, count - 1} & set(range(count))):
+        q = qs[i % 2]
+        mul = lambda a, b: oracle.mul(a[i], b[i], q, 2)
+        c0, c1, d0, d1 = x
+        for k, exp in enumerate((mul(c0, d0), oracle.add(mul(c0, d1), mul(c1, d0), q), mul(c1, d1))):
+            np.testing.assert_array_equal(got[k][i], exp, err_msg=f"limb {i} output {k}")
