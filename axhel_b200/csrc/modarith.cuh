@@ -30,9 +30,11 @@ __device__ __forceinline__ uint64_t reduce_input(uint64_t x, uint64_t q)
 }
 
 // Conditional subtract for the NTT's bounded ranges: the same function as
-// csub() whenever |x - bound| < 2^63, which holds for every value a transform
-// handles (x < 4q, bound <= 2q, q < 2^62).  Testing the sign of the
-// difference takes one compare on its high word instead of a 64-bit compare.
+// csub() whenever bound <= 2^63 and x - bound < 2^63, which holds for every
+// value a transform handles: x < 4q and bound <= 2q with q < 2^62 in the
+// reference's butterflies, x < 32q and bound <= 16q with q < 2^59 in the relaxed
+// ones.  Testing the sign of the difference takes one compare on its high word
+// instead of a 64-bit compare.
 __device__ __forceinline__ uint64_t csub_lazy(uint64_t x, uint64_t bound)
 {
     const uint64_t d = x - bound;
@@ -149,9 +151,10 @@ __device__ __forceinline__ void inv_final_butterfly(uint64_t& x, uint64_t& y, ui
 // ------------------------------------------------- relaxed integer forms
 // For transforms whose outputs are reduced to [0, q), so that intermediate
 // values may be any representative.  Bound: the integer multiply pipe, where
-// a high 32-bit product costs two low ones; leaving out the low-by-low term of
-// the quotient and its carries takes the butterfly from 40 to 33 clocks per
-// warp on the register-only probe (q of 58 bits).
+// a high 32-bit product costs two low ones; the low-by-low term of the quotient
+// and its carries are left out.  768 limbs of N = 2^16 to [0, q): 60-bit moduli
+// with the reference's butterflies 567 us forward and 599 inverse, 55-bit ones
+// relaxed 530 and 537.
 
 // value * w - e * q with e = floor(value * w' / 2^64) - {0, 1, 2}: the terms
 // y1 w'1, floor(y1 w'0 / 2^32) and floor(y0 w'1 / 2^32) only, each floor and
@@ -178,10 +181,14 @@ __device__ __forceinline__ uint64_t shoup_relaxed(uint64_t v, uint64_t w, uint64
 
 // ---------------------------------------------------------- FP64 forms
 // For q < 2^50.  Residues are integers held in doubles; every value stays
-// below 2^53 in magnitude and every result is an exact integer.  A butterfly
-// is eight FP64 instructions of two clocks each per warp (the FP64 pipe runs
-// at half the FP32 rate and is otherwise idle here) against 36 clocks of
-// integer multiplies: 17-19 clocks against 40 on the register-only probe.
+// below 2^53 in magnitude and every result is an exact integer.  The product is
+// the fused multiply-add one of J. van der Hoeven, G. Lecerf and G. Quintin,
+// "Modular SIMD arithmetic in Mathemagix" (ACM Trans. Math. Softw. 43, 2016): high
+// and low part, a rounded quotient, the remainder.  A butterfly is eight FP64
+// instructions of two clocks each per warp (the FP64 pipe runs at half the FP32
+// rate and is otherwise idle here) against 36 clocks of integer multiplies.  768
+// limbs of N = 2^16 to [0, q), 45-bit moduli: 345 us each way (60 bits, integer:
+// 567 forward, 599 inverse).
 
 constexpr double kFpRound = 6755399441055744.0;  // 1.5 * 2^52: adding it rounds to an integer
 constexpr double kFp2p52 = 4503599627370496.0;

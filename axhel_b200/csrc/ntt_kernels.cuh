@@ -399,6 +399,7 @@ __device__ __forceinline__ double fp_exact_lazy(double y, const ulonglong2 w, ui
 // 192 limbs of N = 2^16).  The FP64 tables therefore hold the 7N/8 entries of
 // those stages (from `tail` on) for 32 neighbouring groups of 8 side by side,
 // one entry of each after the other: fp_tail_pos.
+//
 // A stage's twiddles: the table and where entry m0 + j lies.  For the FP64
 // modes the second word is w / q from the rounded 1/q (relative error 2^-52):
 // one FP64 product for each twiddle, shared by its butterflies, instead of
@@ -977,8 +978,8 @@ __global__ void __launch_bounds__(max_threads(LR), LR == 3 ? 2 : 1) ntt_pass_ker
     uint64_t limb, lstep;
     uint32_t til;
     if (!cta_tile<1>(a, a.logn - LG - lgtg, limb, til, lstep)) return;
-    pass_tile<INV, LG, LR, false, false, true, RELAX, 1, SHAPE>(a.src, a.dst, a.ctx[blockIdx.y], a.logn, a.s0, lgtg, limb, til,
-                                                         a.flags, sm, nullptr, lstep);
+    pass_tile<INV, LG, LR, false, false, true, RELAX, 1, SHAPE>(
+        a.src, a.dst, a.ctx[blockIdx.y], a.logn, a.s0, lgtg, limb, til, a.flags, sm, nullptr, lstep);
 }
 
 // Sixteen registers of the limb per thread: held to the machine registers it
@@ -991,8 +992,8 @@ __global__ void __maxnreg__(INV ? 80 : 72) ntt_pass16_kernel(const __grid_consta
     uint64_t limb, lstep;
     uint32_t til;
     if (!cta_tile<1>(a, a.logn - LG - lgtg, limb, til, lstep)) return;
-    pass_tile<INV, LG, 4, false, false, true, false, 1, SHAPE>(a.src, a.dst, a.ctx[blockIdx.y], a.logn, a.s0, lgtg, limb, til,
-                                                         a.flags, sm, nullptr, lstep);
+    pass_tile<INV, LG, 4, false, false, true, false, 1, SHAPE>(
+        a.src, a.dst, a.ctx[blockIdx.y], a.logn, a.s0, lgtg, limb, til, a.flags, sm, nullptr, lstep);
 }
 
 template <bool INV, int LG, int LR, bool RELAX, int SHAPE>
@@ -1003,8 +1004,8 @@ __global__ void __maxnreg__(kPairRegs) ntt_pass_pair_kernel(const __grid_constan
     uint64_t limb, lstep;
     uint32_t til;
     if (!cta_tile<2>(a, a.logn - LG - lgtg, limb, til, lstep)) return;
-    pass_tile<INV, LG, LR, false, false, true, RELAX, 2, SHAPE>(a.src, a.dst, a.ctx[blockIdx.y], a.logn, a.s0, lgtg, limb, til,
-                                                         a.flags, sm, nullptr, lstep);
+    pass_tile<INV, LG, LR, false, false, true, RELAX, 2, SHAPE>(
+        a.src, a.dst, a.ctx[blockIdx.y], a.logn, a.s0, lgtg, limb, til, a.flags, sm, nullptr, lstep);
 }
 
 // The same pass with the dyadic product of kPreMul / kPostMul: a kernel of
@@ -1018,8 +1019,8 @@ __global__ void __launch_bounds__(max_threads(LR), LR == 3 ? 2 : 1) ntt_pass_mul
     uint64_t limb, lstep;
     uint32_t til;
     if (!cta_tile<1>(a, a.logn - LG - lgtg, limb, til, lstep)) return;
-    pass_tile<INV, LG, LR, false, true, true, RELAX, 1, SHAPE>(a.src, a.dst, a.ctx[blockIdx.y], a.logn, a.s0, lgtg, limb, til,
-                                                        a.flags, sm, a.operand, lstep);
+    pass_tile<INV, LG, LR, false, true, true, RELAX, 1, SHAPE>(
+        a.src, a.dst, a.ctx[blockIdx.y], a.logn, a.s0, lgtg, limb, til, a.flags, sm, a.operand, lstep);
 }
 
 template <bool INV, int LG, int SHAPE>
@@ -1030,8 +1031,8 @@ __global__ void __maxnreg__(128) ntt_pass_mul16_kernel(const __grid_constant__ P
     uint64_t limb, lstep;
     uint32_t til;
     if (!cta_tile<1>(a, a.logn - LG - lgtg, limb, til, lstep)) return;
-    pass_tile<INV, LG, 4, false, true, true, false, 1, SHAPE>(a.src, a.dst, a.ctx[blockIdx.y], a.logn, a.s0, lgtg, limb, til,
-                                                        a.flags, sm, a.operand, lstep);
+    pass_tile<INV, LG, 4, false, true, true, false, 1, SHAPE>(
+        a.src, a.dst, a.ctx[blockIdx.y], a.logn, a.s0, lgtg, limb, til, a.flags, sm, a.operand, lstep);
 }
 
 template <bool INV, int LG, int LR, bool RELAX, int SHAPE>
@@ -1042,8 +1043,8 @@ __global__ void __maxnreg__(kPairRegs) ntt_pass_mul_pair_kernel(const __grid_con
     uint64_t limb, lstep;
     uint32_t til;
     if (!cta_tile<2>(a, a.logn - LG - lgtg, limb, til, lstep)) return;
-    pass_tile<INV, LG, LR, false, true, true, RELAX, 2, SHAPE>(a.src, a.dst, a.ctx[blockIdx.y], a.logn, a.s0, lgtg, limb, til,
-                                                        a.flags, sm, a.operand, lstep);
+    pass_tile<INV, LG, LR, false, true, true, RELAX, 2, SHAPE>(
+        a.src, a.dst, a.ctx[blockIdx.y], a.logn, a.s0, lgtg, limb, til, a.flags, sm, a.operand, lstep);
 }
 
 // Fused column pass of an INTT -> op -> NTT chain: the inverse's last pass
@@ -1127,7 +1128,7 @@ __device__ __forceinline__ void chain_tile_as(const uint64_t* src, uint64_t* dst
 #pragma unroll
                 for (int i = 0; i < R; ++i) {
                     double x = fp_reduce(as_fp(v[p][i]), fq, fqi);
-                        if (__double2hiint(x) < 0) x = __dadd_rn(x, fq);
+                    if (__double2hiint(x) < 0) x = __dadd_rn(x, fq);
                     v[p][i] = as_u64(x);
                 }
             }
@@ -1296,7 +1297,8 @@ __global__ void __maxnreg__(product_regs(P)) ntt_product_kernel(const __grid_con
     uint64_t limb, lstep;
     uint32_t til;
     if (!cta_tile<P>(a, a.logn - LG - lgtg, limb, til, lstep)) return;
-    product_tile<LG, LR, MODES, RELAX, P>(a.src, a.dst, c.operand, a.ctx[blockIdx.y], a.logn, lgtg, limb, lstep, til, a.flags, sm);
+    product_tile<LG, LR, MODES, RELAX, P>(a.src, a.dst, c.operand, a.ctx[blockIdx.y], a.logn, lgtg, limb, lstep, til,
+                                          a.flags, sm);
 }
 
 // Kernel of the fused chain pass: one CTA per tile of chain_tile above; the
@@ -1310,8 +1312,8 @@ __global__ void __maxnreg__(chain_regs(LR)) ntt_chain_kernel(const __grid_consta
     uint64_t limb, lstep;
     uint32_t til;
     if (!cta_tile<P>(a, a.logn - LG - lgtg, limb, til, lstep)) return;
-    chain_tile<LG, LR, false, MODES, RELAX, P>(a.src, a.dst, c.operand, a.ctx[blockIdx.y], c.op, c.scalar[blockIdx.y], a.logn, lgtg,
-                                              limb, til, a.flags, sm, lstep);
+    chain_tile<LG, LR, false, MODES, RELAX, P>(a.src, a.dst, c.operand, a.ctx[blockIdx.y], c.op, c.scalar[blockIdx.y],
+                                               a.logn, lgtg, limb, til, a.flags, sm, lstep);
 }
 
 }  // namespace axhel_impl

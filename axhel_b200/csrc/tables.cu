@@ -71,7 +71,8 @@ __global__ void __launch_bounds__(256) gen_tables_kernel(const __grid_constant__
     const uint64_t r = mont_mul(w, j.r2m, j.q, j.mninv);     // w 2^64 mod q
     *out = make_ulonglong2(w, r * j.mninv);                  // Q = (w 2^64 - r) / q
     if (j.hdr.arith == 2) {
-        double* fout = const_cast<double*>(inv ? j.hdr.finv : j.hdr.ffwd) + (i ? fp_table_pos(inv, i, (uint32_t)n, j.logn) : 0);
+        const uint32_t at = i ? fp_table_pos(inv, i, (uint32_t)n, j.logn) : 0;
+        double* fout = const_cast<double*>(inv ? j.hdr.finv : j.hdr.ffwd) + at;
         *fout = (double)(w > (j.q >> 1) ? (int64_t)(w - j.q) : (int64_t)w);
     }
 }
