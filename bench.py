@@ -303,8 +303,10 @@ def run_ours(args):
                     "traffic": traffic, "kernel": name, "launches": cnt, "avg_launch_ms": tot / cnt,
                     "alg_bytes_per_launch": alg, "peak_source": f"{peak_kind} hbm_gbs",
                     "share": tot / sum(v[1] for v in prof.values())}
-        # The binding roofline is the integer pipe: butterflies of the
-        # reference algebra per second against the register-only probe.
+        # The binding roofline is the integer pipe: butterflies per second
+        # against the register-only probe of the reference's butterfly, which
+        # the lazy forward runs (the inverse's relaxed and FP64 ones need fewer
+        # multiplies, so step_frac compares rates and is no share of a ceiling).
         lg = int(name.split("lg=")[1].split()[0])
         bfly_launch = COUNT * (N // 2) * lg
         bpeak = max(capi.butterfly_peak(ntts[0], False, sh) for _ in range(3))
