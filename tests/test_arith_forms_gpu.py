@@ -174,3 +174,37 @@ def test_tensor_without_fp64_moduli(cuda, oracle, n, count):
         c0, c1, d0, d1 = x
         for k, exp in enumerate((mul(c0, d0), oracle.add(mul(c0, d1), mul(c1, d0), q), mul(c1, d1))):
             np.testing.assert_array_equal(got[k][i], exp, err_msg=f"limb {i} output {k}")
+
+
+def sparse_inputs(rng, n, q):
+    """Zeros, a constant, polynomials in X^2 and X^4, a zero upper half, multiples of q, small values."""
+    x = np.zeros((8, n), np.uint64)
+    x[1, 0] = q - 1
+    x[2, ::2] = rng.integers(0, q, n // 2, dtype=np.uint64)
+    x[3, ::4] = rng.integers(0, 4 * q, n // 4, dtype=np.uint64)
+    x[4, : n // 2] = rng.integers(0, q, n // 2, dtype=np.uint64)
+    x[5] = q * rng.integers(0, 4, n).astype(np.uint64)
+    x[6] = rng.integers(0, 3, n, dtype=np.uint64)
+    x[7] = np.where(rng.integers(0, 2, n) == 0, 0, rng.integers(0, 4 * q, n, dtype=np.uint64))
+    return x
+
+
+# enough residues for the FP64 form of a lazy forward
+@pytest.mark.parametrize("n,copies", [(64, 768), (4096, 13), (16384, 4), (65536, 1)])
+@pytest.mark.parametrize("bits,num,den", [(20, 1, 2), (30, 1, 2), (45, 1, 2), (50, 1, 1)])
+def test_lazy_forward_of_sparse_inputs(cuda, oracle, n, copies, bits, num, den):
+    q = oracle.find_ntt_prime_near(n, bits, num, den)
+    psi = oracle.find_primitive_root(n, q)
+    t = cuda.NTT(n, q, psi)
+    fwd, inv, ninv = oracle.tables(n, q, psi)
+    rng = np.random.default_rng(n + bits)
+    x = sparse_inputs(rng, n, q)
+    x2, m = x % np.uint64(2 * q), rng.integers(0, 2 * q, n, dtype=np.uint64)
+    count = len(x) * copies
+    d, d2, e, o = dev(np.tile(x, (copies, 1))), dev(np.tile(x2, (copies, 1))), dev(np.tile(m, count)), dev_empty(count * n)
+    cuda.forward_batch([t], ptr(o), ptr(d), count, 4, 4)
+    want = np.stack([oracle.forward(v, q, fwd, 4, 4) for v in x])
+    np.testing.assert_array_equal(host(o).reshape(copies, len(x), n), np.broadcast_to(want, (copies, len(x), n)))
+    cuda.chain_mul_batch([t], ptr(o), ptr(d2), ptr(e), count, 2, 4)
+    want = np.stack([oracle.forward(oracle.mul(oracle.inverse(v, q, inv, ninv, 2, 2), m, q, 2), q, fwd, 1, 4) for v in x2])
+    np.testing.assert_array_equal(host(o).reshape(copies, len(x), n), np.broadcast_to(want, (copies, len(x), n)))
