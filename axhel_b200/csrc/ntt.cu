@@ -77,15 +77,14 @@ cudaError_t launch_tiles(const FnTable<void (*)(const Args)>& t, FnKind kind, bo
     const unsigned threads = (unsigned)c.tg << (c.lg - c.lr);
     count_launch();
     // A last group that holds only some of the moduli: the CTAs of its missing
-    // limbs would lie between the others and leave SMs idle.  Few limbs are
+    // limbs would lie between the others and leave SMs idle, so few limbs are
     // launched as one group, each with its own context (N = 2^16, 55 bits, us:
     // 9 limbs of 8 moduli forward 13.7 to 10.7, product 30.6 to 22.1; 32 of 24
-    // 28.9 to 25.9, 67.9 to 64.1); otherwise the groups go to blockIdx.z, which
-    // puts those CTAs last (300 limbs of 24 moduli of 2^13: 28.2 to 26.4, 60.2 to
-    // 56.0).
+    // 28.9 to 25.9, 67.9 to 64.1).  (More limbs with the groups in blockIdx.z,
+    // which puts the missing ones last: 2-7 % faster, 300 of 24 of 2^13 28.2 to
+    // 26.4, but the index costs canonical forwards of full groups 1 %.)
     const uint64_t moduli = pass.count < pass.nctx ? pass.count : pass.nctx;
-    const bool partial = pass.count % moduli != 0;
-    if (partial && !pair && pass.count <= (uint64_t)kMaxInlineMods) {
+    if (pass.count % moduli != 0 && !pair && pass.count <= (uint64_t)kMaxInlineMods) {
         Args one = args;
         PassArgs& p = pass_of(one);
         p.nctx = (uint32_t)pass.count;
@@ -96,10 +95,8 @@ cudaError_t launch_tiles(const FnTable<void (*)(const Args)>& t, FnKind kind, bo
         fn<<<dim3((unsigned)per_limb, p.nctx), threads, smem_bytes(c), s>>>(one);
         return cudaGetLastError();
     }
-    const uint64_t groups = (pass.count + moduli - 1) / moduli, gs = (groups + pair) >> pair;
-    const bool in_z = partial && gs <= 65535;
-    const dim3 grid((unsigned)(in_z ? per_limb : gs * per_limb), (unsigned)moduli, in_z ? (unsigned)gs : 1);
-    fn<<<grid, threads, smem_bytes(c) << pair, s>>>(args);
+    const uint64_t groups = (pass.count + moduli - 1) / moduli, gx = ((groups + pair) >> pair) * per_limb;
+    fn<<<dim3((unsigned)gx, (unsigned)moduli), threads, smem_bytes(c) << pair, s>>>(args);
     return cudaGetLastError();
 }
 

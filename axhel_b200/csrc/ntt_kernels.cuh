@@ -972,10 +972,9 @@ __device__ __forceinline__ void pass_tile(const uint64_t* src, uint64_t* dst, co
     });
 }
 
-// CTA -> tile: blockIdx.y is the modulus, blockIdx.x the tile in the limb and,
-// above it, or in blockIdx.z, the group of nctx limbs (with P = 2 the pair of
-// groups).  (No division, and the modulus context is uniform over the CTA for
-// the compiler too.)  `lstep`:
+// CTA -> tile: blockIdx.y is the modulus, blockIdx.x the group of nctx limbs
+// (with P = 2 the pair of groups) and the tile in the limb.  (No division, and
+// the modulus context is uniform over the CTA for the compiler too.)  `lstep`:
 // the distance to the second limb of a pair, 0 for a limb without a partner,
 // which is then its own (both copies hold the same values and write them to
 // the same place).
@@ -984,7 +983,7 @@ __device__ __forceinline__ bool cta_tile(const PassArgs& a, uint32_t lg_tiles, u
                                          uint64_t& lstep)
 {
     tile_in_limb = blockIdx.x & ((1u << lg_tiles) - 1);
-    limb = ((uint64_t)(blockIdx.x >> lg_tiles) + blockIdx.z) * P * a.nctx + blockIdx.y;
+    limb = (uint64_t)(blockIdx.x >> lg_tiles) * P * a.nctx + blockIdx.y;
     lstep = P == 1 || limb + a.nctx >= a.count ? 0 : a.nctx;
     return limb < a.count;
 }
