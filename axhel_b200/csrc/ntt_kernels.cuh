@@ -449,10 +449,12 @@ __device__ __forceinline__ StageTw stage_tw(const ModArith& a, uint32_t nat, uin
 // is that small recomputes those products with the integer formula.  A zero
 // remainder needs none: y = 0 gives t = 0, and y = kq, k = 1..3, gives y w' =
 // k (w 2^64 - (w 2^64 mod q)), whose quotient is kw - 1, so t = q.  (Zeros become
-// such multiples in the first stage, x + t and x + 2q - t: 768 limbs of N = 2^16
-// with every second coefficient zero take 590 us, 884 with the integer formula for
-// each; 480 without zeros, 551 with the reference's butterflies whatever the
-// values.)
+// such multiples in the first stage, x + t and x + 2q - t.  768 limbs of N = 2^16,
+// 45 bits: 499 us whatever the values; with the integer formula for every zero
+// remainder 480 for values without any and 884-948 for zeros, every second
+// coefficient zero or multiples of q; with a second look at them after the check
+// 478 and 590, but 2 % more for the wide moduli that share the kernel.  The
+// reference's butterflies: 551.)
 template <int MODE, int LG, int LR, int RD, int P>
 __device__ __forceinline__ void fwd_stages(uint64_t (&v)[P][1 << LR], uint32_t rbase, uint32_t blk, uint32_t s0,
                                            const ModArith& a)
@@ -472,7 +474,7 @@ __device__ __forceinline__ void fwd_stages(uint64_t (&v)[P][1 << LR], uint32_t r
         const StageTw tw = stage_tw<MODE>(a, 1u << t, m0, b, a.n >> 3);
         if constexpr (MODE == kFpLazy) {
             double r[P][R / 2];
-            uint32_t least = 0xffffffffu;
+            uint32_t least = 0xffffffffu;  // high word of the least remainder but zero, less 1
 #pragma unroll
             for (int j = 0; j < (R >> (rb + 1)); ++j) {
                 const ulonglong2 w = tw.get<MODE>(j, b, a.fqi);
@@ -481,34 +483,23 @@ __device__ __forceinline__ void fwd_stages(uint64_t (&v)[P][1 << LR], uint32_t r
 #pragma unroll
                     for (int l = 0; l < (1 << rb); ++l) {
                         const int k = (j << rb) | l, i1 = (j << (rb + 1)) | l | (1 << rb);
-                        double x = fp_mul(as_fp(v[p][i1]), as_fp(w.x), as_fp(w.y), a.fq);
-                        if (__double2hiint(x) < 0) x = __dadd_rn(x, a.fq);
+                        const double y = as_fp(v[p][i1]);
+                        double x = fp_mul(y, as_fp(w.x), as_fp(w.y), a.fq);
+                        // negative, or zero with y not (only zero has a zero high word)
+                        if (__double2hiint(x) < min(__double2hiint(y), 1)) x = __dadd_rn(x, a.fq);
                         r[p][k] = x;
-                        least = min(least, (uint32_t)__double2hiint(x));
+                        least = __viaddmin_u32((uint32_t)__double2hiint(x), 0xffffffffu, least);
                     }
             }
-            if (least <= a.lazy_hi) {
-                // zero remainders first (only zero has a zero high word)
-                least = 0xffffffffu;
+            if (least < a.lazy_hi) {
 #pragma unroll
                 for (int p = 0; p < P; ++p)
 #pragma unroll
                     for (int k = 0; k < R / 2; ++k) {
-                        const int i1 = ((k >> rb) << (rb + 1)) | (k & ((1 << rb) - 1)) | (1 << rb);
-                        const uint32_t h = (uint32_t)__double2hiint(r[p][k]);
-                        if (h == 0 && __double2hiint(as_fp(v[p][i1])) != 0) r[p][k] = a.fq;
-                        least = min(least, h - 1);
+                        const int j = k >> rb, i1 = (j << (rb + 1)) | (k & ((1 << rb) - 1)) | (1 << rb);
+                        if ((uint32_t)__double2hiint(r[p][k]) - 1 < a.lazy_hi)
+                            r[p][k] = fp_exact_lazy(as_fp(v[p][i1]), twiddle(a.itw, (1u << t) + m0 + j), a.q);
                     }
-                if (least < a.lazy_hi) {
-#pragma unroll
-                    for (int p = 0; p < P; ++p)
-#pragma unroll
-                        for (int k = 0; k < R / 2; ++k) {
-                            const int j = k >> rb, i1 = (j << (rb + 1)) | (k & ((1 << rb) - 1)) | (1 << rb);
-                            if ((uint32_t)__double2hiint(r[p][k]) - 1 < a.lazy_hi)
-                                r[p][k] = fp_exact_lazy(as_fp(v[p][i1]), twiddle(a.itw, (1u << t) + m0 + j), a.q);
-                        }
-                }
             }
             const double q2 = __dadd_rn(a.fq, a.fq);
 #pragma unroll
